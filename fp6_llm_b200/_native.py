@@ -16,7 +16,7 @@ _CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libfp6_b200.so")
 SOURCES = ("fpx_gemm.cu", "fpx_native.cu", "fpx_prepack.cu", "c_api.cu", "c_api_noalloc.cu")
-HEADERS = ("fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
+HEADERS = ("fpx_codes.cuh", "fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--threads", "4",
               "-Xcompiler", "-fPIC", "-shared"]
@@ -27,7 +27,7 @@ C_SYMBOLS = (
     "fp6b200_workspace_bytes", "fp6b200_choose_split_k", "fp6b200_prepack", "fp6b200_prepack_host",
     "fp6b200_dequant", "fp6b200_dequant_host", "fp6b200_dequant_packed", "fp6b200_splitk_reduce",
     "fp6b200_device_status", "fp6b200_linear_static_scratch", "fp6b200_static_scratch_bytes",
-    "fp6b200_linear_gather", "fp6b200_set_option", "fp6b200_get_option", "fp6b200_quantize_prepack",
+    "fp6b200_linear_gather", "fp6b200_set_option", "fp6b200_get_option", "fp6b200_quantize_prepack", "fp6b200_row_scales",
     "fp6b200_linear_host_io_batch", "fp6b200_kernel_launches", "fp6b200_linear_ex",
     "fp6b200_native_supported", "fp6b200_native_preferred", "fp6b200_native_weight_bytes", "fp6b200_native_workspace_bytes",
     "fp6b200_native_repack", "fp6b200_linear_native", "fp6b200_native_kernel_launches", "fp6b200_linear_native_gather",
@@ -145,6 +145,8 @@ def lib() -> ctypes.CDLL:
     L.fp6b200_get_option.argtypes = [ci]
     L.fp6b200_quantize_prepack.restype = ci
     L.fp6b200_quantize_prepack.argtypes = [ci, ci, vp, vp, vp, vp, sz, sz]
+    L.fp6b200_row_scales.restype = ci
+    L.fp6b200_row_scales.argtypes = [vp, vp, vp, sz, sz, ctypes.c_float]
     L.fp6b200_device_status.restype = ci
     L.fp6b200_device_status.argtypes = [ctypes.POINTER(ci)]
     _lib = L

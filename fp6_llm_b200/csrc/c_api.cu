@@ -368,6 +368,11 @@ int fp6b200_quantize_prepack(int e_bits, int m_bits, void* stream, const void* w
                                         packed_dev, M, K);
 }
 
+int fp6b200_row_scales(void* stream, const void* weights_fp16_dev, void* scales_dev, size_t M, size_t K, float top) {
+    return fpx::launch_row_scales(static_cast<cudaStream_t>(stream), static_cast<const __half*>(weights_fp16_dev),
+                                  static_cast<__half*>(scales_dev), M, K, top);
+}
+
 int fp6b200_prepack_host(int e_bits, int m_bits, int* packed_host, const int* unpacked_host, size_t M, size_t K) {
     if (!fpx::format_supported(e_bits, m_bits) || !packed_host || !unpacked_host || M % 64 || K % 64 || !M || !K)
         return cudaErrorInvalidValue;

@@ -114,6 +114,8 @@ cudaError_t launch_prepack(int e_bits, int m_bits, cudaStream_t stream, const vo
 // fp16 weights [M][K] + fp16 row scales -> prepacked FPx (round to nearest, ties to the even code, saturating).
 cudaError_t launch_quantize_prepack(int e_bits, int m_bits, cudaStream_t stream, const __half* weights,
                                     const __half* scales, void* packed, size_t M, size_t K);
+// scales[m] = max|w[m][:]| / top, at least 2^-24, as fp16 (K a multiple of 8, weights 16-byte aligned).
+cudaError_t launch_row_scales(cudaStream_t stream, const __half* weights, __half* scales, size_t M, size_t K, float top);
 cudaError_t launch_dequant_unpacked(int e_bits, int m_bits, cudaStream_t stream, const void* unpacked,
                                     const __half* scales, __half* out, size_t M, size_t K);
 cudaError_t launch_dequant_packed(int e_bits, int m_bits, cudaStream_t stream, const void* packed,

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fpx_codes.cuh"
 #include "fpx_internal.h"
 #include "fpx_layout.h"
 
@@ -75,55 +76,173 @@ prepack_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32
 // Round-to-nearest quantiser fused with the packer: fp16 weights [M, K] and fp16 row scales in, prepacked FPx out,
 // without the unpacked tensor in between.  (The reference ships no working quantiser: fp6_llm/csrc/utils/
 // weight_quant.h:9-104 truncates and is not bound; the layout it would feed is the packer's above.)
-// Code of a weight = nearest representable magnitude of |w / scale| (the division in fp32, round to nearest);
-// ties go to the even code; beyond the largest magnitude it saturates; the sign bit is the sign of the quotient.
+// Code of a weight = nearest representable magnitude of |w / scale|; ties go to the even code; beyond the largest
+// magnitude it saturates; the sign bit is the sign of the quotient.
+//
+// HBM-bound (2 + bw / 8 bytes per weight), so the instructions per weight have to stay near ten.  The exact definition
+// (quantize_rtn_code: a division and a compare with every midpoint) took 8660 us on 8192 x 28672 e3m2 weights; this form
+// takes 113 us = 5.7 TB/s:
+//   * w * (1 / scale), with the reciprocal taken once per row, instead of w / scale.  Only the side of the quotient on which
+//     a midpoint lies matters, and for fp16 w and scale the two are equal or at least 2^-16 (relative) apart: w and midpoint *
+//     scale are integers below 2^11 and 2^16 in units of a power of two.  The product is within 2^-22 of the quotient, so
+//     rounding it to a multiple of 32 units in the last place (2^-18) puts exact ties back on the midpoint, which has at most
+//     five significant bits, and moves nothing else across one.
+//   * rounding to the format by cvt for e3m2 and e2m3, by one addition of a power of two otherwise (round_code).
+//   * a lane reads 16 bytes of a row; the packed words are put together in registers (fpx_codes.cuh).
+// Rows whose scale is zero, negative or not finite, and chunks that hold an infinite or NaN weight, take the exact definition.
+constexpr int kQuantWarps = 8;
+constexpr int kQuantSlots = 2;     // 32-column units per warp: one reciprocal per row and 512 columns
+
+// Code of the magnitude and sign in the bits of a finite float: 2^(23 - M) times the binade's unit (at least the subnormals'
+// binade) is added, so that the addition itself rounds to the format's last bit, ties to even.
 template <int E_BITS, int M_BITS>
-__global__ void __launch_bounds__(kPrepackThreads)
+__device__ __forceinline__ uint32_t round_code(uint32_t u) {
+    constexpr int kBias = (1 << (E_BITS - 1)) - 1;
+    constexpr uint32_t kMinBinade = (uint32_t)(127 + 1 - kBias) << 23;
+    // the largest magnitude: (2 - 2^-M) * 2^(2^E - 1 - bias)
+    constexpr uint32_t kTop = ((uint32_t)(127 + (1 << E_BITS) - 1 - kBias) << 23) | (((1u << M_BITS) - 1u) << (23 - M_BITS));
+    const uint32_t a = min(u & 0x7fffffffu, kTop);
+    const uint32_t binade = max(a & 0x7f800000u, kMinBinade);
+    const uint32_t c = binade + ((uint32_t)(23 - M_BITS) << 23);
+    const uint32_t t = __float_as_uint(__uint_as_float(a) + __uint_as_float(c));
+    return (t - c) + ((binade - kMinBinade) >> (23 - M_BITS)) + ((u >> 31) << (E_BITS + M_BITS));
+}
+
+// Eight codes, one per byte, of q[0..7].
+template <int E_BITS, int M_BITS>
+__device__ __forceinline__ void round_codes8(const float (&q)[8], uint32_t& lo, uint32_t& hi) {
+    uint32_t u[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) u[i] = (__float_as_uint(q[i]) + 16u) & 0xffffffe0u;
+    if constexpr ((E_BITS == 3 && M_BITS == 2) || (E_BITS == 2 && M_BITS == 3)) {
+        uint32_t pair[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float even = __uint_as_float(u[2 * i]), odd = __uint_as_float(u[2 * i + 1]);
+            uint16_t h;
+            if constexpr (E_BITS == 3) asm("cvt.rn.satfinite.e3m2x2.f32 %0, %1, %2;" : "=h"(h) : "f"(odd), "f"(even));
+            else asm("cvt.rn.satfinite.e2m3x2.f32 %0, %1, %2;" : "=h"(h) : "f"(odd), "f"(even));
+            pair[i] = h;
+        }
+        lo = pair[0] | (pair[1] << 16);
+        hi = pair[2] | (pair[3] << 16);
+    } else {
+        uint32_t c[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) c[i] = round_code<E_BITS, M_BITS>(u[i]);
+        lo = c[0] | (c[1] << 8) | (c[2] << 16) | (c[3] << 24);
+        hi = c[4] | (c[5] << 8) | (c[6] << 16) | (c[7] << 24);
+    }
+}
+
+template <int E_BITS, int M_BITS>
+__device__ __noinline__ uint2 exact_codes8(uint4 raw, float scale) {
+    const uint32_t h[4] = {raw.x, raw.y, raw.z, raw.w};
+    uint32_t out[2] = {0u, 0u};
+    for (int i = 0; i < 8; i++) {
+        const float w = __half2float(__ushort_as_half((unsigned short)(h[i >> 1] >> (16 * (i & 1)))));
+        out[i >> 2] |= quantize_rtn_code(E_BITS, M_BITS, __fdiv_rn(w, scale)) << (8 * (i & 3));
+    }
+    return make_uint2(out[0], out[1]);
+}
+
+template <int E_BITS, int M_BITS>
+__global__ void __launch_bounds__(kQuantWarps * 32)
 quantize_prepack_kernel(const __half* __restrict__ w, const __half* __restrict__ scales, uint8_t* __restrict__ out,
-                        uint32_t M, uint32_t K) {
+                        uint32_t K, uint32_t ctas_per_row, uint64_t off2, uint64_t off4, int aligned16) {
     constexpr int BW = 1 + E_BITS + M_BITS;
-    constexpr uint32_t kCols = kChunkKBlocks * kKBlock;
-    constexpr uint32_t kPitch = kCols + 4;
-    __shared__ __align__(16) uint8_t codes[kRowsPerBlock * kPitch];
-
-    const uint32_t kblocks = K / kKBlock;
-    const uint32_t chunks_per_row = (kblocks + kChunkKBlocks - 1) / kChunkKBlocks;
-    const uint32_t i = blockIdx.x / chunks_per_row;            // 64-row block
-    const uint32_t kb0 = (blockIdx.x % chunks_per_row) * kChunkKBlocks;
-    const uint32_t nkb = min((uint32_t)kChunkKBlocks, kblocks - kb0);
-    const uint32_t ncols = nkb * kKBlock;
-    const uint32_t col0 = kb0 * kKBlock;
-
-    for (uint32_t x = threadIdx.x; x < kRowsPerBlock * (ncols / 2); x += kPrepackThreads) {   // two weights per thread and round
-        const uint32_t r = x / (ncols / 2), c = (x % (ncols / 2)) * 2;
-        const uint32_t row = i * kRowsPerBlock + r;
-        const __half2 pair = *reinterpret_cast<const __half2*>(w + (size_t)row * K + col0 + c);
-        const float sc = __half2float(scales[row]);
-        codes[r * kPitch + c] = (uint8_t)quantize_rtn_code(E_BITS, M_BITS, __fdiv_rn(__low2float(pair), sc));
-        codes[r * kPitch + c + 1] = (uint8_t)quantize_rtn_code(E_BITS, M_BITS, __fdiv_rn(__high2float(pair), sc));
+    __shared__ float row_scale[kRowsPerBlock], row_inv[kRowsPerBlock];   // row_inv 0: the row takes the exact definition
+    const uint32_t i = blockIdx.x / ctas_per_row;              // 64-row block
+    const uint32_t first_unit = (blockIdx.x - i * ctas_per_row) * kQuantSlots * kQuantWarps;
+    const int lane = threadIdx.x & 31, g = lane >> 2, s = lane & 3;
+    if (threadIdx.x < kRowsPerBlock) {
+        const float sc = __half2float(scales[(size_t)i * kRowsPerBlock + threadIdx.x]);
+        row_scale[threadIdx.x] = sc;
+        row_inv[threadIdx.x] = (sc > 0.0f && sc < 65536.0f) ? 1.0f / sc : 0.0f;
     }
     __syncthreads();
-
+    const uint32_t units = K / 32;
+#pragma unroll 1
+    for (int slot = 0; slot < kQuantSlots; slot++) {
+        const uint32_t unit = first_unit + slot * kQuantWarps + (threadIdx.x >> 5);
+        if (unit >= units) return;
+        const __half* src = w + ((size_t)i * kRowsPerBlock + g) * K + (size_t)unit * 32 + s * 8;
+        uint4 raw[8];
 #pragma unroll
-    for (int wd = 1; wd <= 4; wd <<= 1) {
-        if (!has_seg(BW, wd)) continue;
-        const int shift = seg_shift(BW, wd);
-        const uint32_t words_per_tile = 4u * wd * 32u;
-        uint32_t* region = reinterpret_cast<uint32_t*>(out + region_offset(BW, wd, M, K));
-        for (uint32_t x = threadIdx.x; x < nkb * words_per_tile; x += kPrepackThreads) {
-            const uint32_t kb = kb0 + x / words_per_tile;
-            const uint32_t in_tile = x % words_per_tile;
-            const int lane = in_tile & 31;
-            const uint64_t word_in_lane = ((uint64_t)i * kblocks + kb) * (4u * wd) + (in_tile >> 5);
-            uint32_t word = 0;
-#pragma unroll 8
-            for (int pos = 0; pos < 32 / wd; pos++) {
-                const FieldSource src = field_source(wd, word_in_lane, lane, pos, K);
-                const uint32_t code = codes[(src.row - i * kRowsPerBlock) * kPitch + (src.col - col0)];
-                word |= ((code >> shift) & ((1u << wd) - 1u)) << (32 - (pos + 1) * wd);
+        for (int r = 0; r < 8; r++) {
+            const __half* p = src + (size_t)(8 * r) * K;
+            if (aligned16) {
+                raw[r] = __ldg(reinterpret_cast<const uint4*>(p));
+            } else {
+                const uint32_t* p4 = reinterpret_cast<const uint32_t*>(p);
+                raw[r] = make_uint4(__ldg(p4), __ldg(p4 + 1), __ldg(p4 + 2), __ldg(p4 + 3));
             }
-            region[word_in_lane * 32 + lane] = word;
         }
+        PackedUnit<BW> words;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            uint32_t lo[2], hi[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const uint4 v = raw[2 * k + r];
+                const int row = 16 * k + 8 * r + g;
+                const float inv = row_inv[row];
+                const __half2* h = reinterpret_cast<const __half2*>(&v);
+                // 0 * x summed over the chunk: anything but a zero means an infinite or NaN weight
+                const __half2 zero = __half2half2(__ushort_as_half((unsigned short)0));
+                const __half2 probe = __hfma2(h[0], zero, __hfma2(h[1], zero, __hfma2(h[2], zero, __hmul2(h[3], zero))));
+                if (inv == 0.0f || (*reinterpret_cast<const uint32_t*>(&probe) & 0x7fff7fffu) != 0u) {
+                    const uint2 c = exact_codes8<E_BITS, M_BITS>(v, row_scale[row]);
+                    lo[r] = c.x; hi[r] = c.y;
+                } else {
+                    float q[8];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float2 f = __half22float2(h[e]);
+                        q[2 * e] = f.x * inv;
+                        q[2 * e + 1] = f.y * inv;
+                    }
+                    round_codes8<E_BITS, M_BITS>(q, lo[r], hi[r]);
+                }
+            }
+            __syncwarp();
+            uint32_t b[4];
+            rows_to_quad_words(lo[0], hi[0], lo[1], hi[1], b);
+            quad_transpose(b, lane);
+            words.add(k, b);
+        }
+        words.store(out, off2, off4, (uint64_t)i * (K / 16) + (uint64_t)unit * 2, lane);
+    }
+}
+
+// Row scales of a quantiser: max|w| of a row divided by the format's largest magnitude, not below 2^-24, as fp16.  One CTA per
+// row, 16 bytes per lane and round.  Absolute values of fp16 compare like their bit patterns, with NaN above infinity, so
+// the maximum is taken on integers and a NaN in the row comes out as NaN.  HBM-bound: 69 us = 6.8 TB/s on
+// 8192 x 28672 (five elementwise and reduction launches in fp32 took 1045 us).
+__global__ void __launch_bounds__(256) row_scales_kernel(const __half* __restrict__ w, __half* __restrict__ scales, uint32_t K,
+                                                          float inv_top) {
+    const uint4* row = reinterpret_cast<const uint4*>(w + (size_t)blockIdx.x * K);
+    const uint32_t chunks = K / 8;
+    uint32_t m = 0;   // two 16-bit maxima
+    auto take = [&](const uint4& v) {
+        m = __vmaxu2(m, __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu)));
+    };
+    uint32_t c = threadIdx.x;
+    for (; c + 3 * 256 < chunks; c += 4 * 256) {   // four loads in flight per lane
+        const uint4 v0 = __ldg(row + c), v1 = __ldg(row + c + 256), v2 = __ldg(row + c + 512), v3 = __ldg(row + c + 768);
+        take(v0); take(v1); take(v2); take(v3);
+    }
+    for (; c < chunks; c += 256) take(__ldg(row + c));
+    m = max(m & 0xffffu, m >> 16);
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ uint32_t part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int i = 1; i < 8; i++) m = max(m, part[i]);
+        const float s = __half2float(__ushort_as_half((unsigned short)m)) * inv_top;
+        scales[blockIdx.x] = __float2half_rn(s < 5.9604644775390625e-8f ? 5.9604644775390625e-8f : s);   // 2^-24; NaN stays
     }
 }
 
@@ -225,11 +344,23 @@ cudaError_t launch_quantize_prepack(int e_bits, int m_bits, cudaStream_t stream,
     if (!shape_ok(e_bits, m_bits, M, K) || !weights || !scales || !packed) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(weights) & 3) || (reinterpret_cast<uintptr_t>(packed) & 3))
         return cudaErrorMisalignedAddress;
-    const size_t kblocks = K / kKBlock;
-    const size_t blocks = (M / kRowsPerBlock) * ((kblocks + kChunkKBlocks - 1) / kChunkKBlocks);
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
     uint8_t* out = static_cast<uint8_t*>(packed);
-    FPX_DISPATCH_FORMAT(e_bits, m_bits, (quantize_prepack_kernel<kE, kM><<<(unsigned)blocks, kPrepackThreads, 0, stream>>>(weights, scales, out, (uint32_t)M, (uint32_t)K)));
+    const int bw = bit_width(e_bits, m_bits);
+    const uint64_t off2 = region_offset(bw, 2, M, K), off4 = region_offset(bw, 4, M, K);
+    const uint32_t units = (uint32_t)(K / 32), per_cta = kQuantWarps * kQuantSlots;
+    const int aligned16 = (reinterpret_cast<uintptr_t>(weights) & 15) == 0;
+    const uint32_t ctas_per_row = (units + per_cta - 1) / per_cta;
+    const size_t blocks = (M / kRowsPerBlock) * ctas_per_row;
+    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    FPX_DISPATCH_FORMAT(e_bits, m_bits, (quantize_prepack_kernel<kE, kM><<<(unsigned)blocks, kQuantWarps * 32, 0, stream>>>(weights, scales, out, (uint32_t)K, ctas_per_row, off2, off4, aligned16)));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_row_scales(cudaStream_t stream, const __half* weights, __half* scales, size_t M, size_t K, float top) {
+    if (!weights || !scales || M == 0 || M > 0x7fffffffull || K == 0 || K % 8 != 0 || K > 0x7fffffffull || !(top > 0.0f))
+        return cudaErrorInvalidValue;
+    if (reinterpret_cast<uintptr_t>(weights) & 15) return cudaErrorMisalignedAddress;
+    row_scales_kernel<<<(unsigned)M, 256, 0, stream>>>(weights, scales, (uint32_t)K, 1.0f / top);
     return cudaGetLastError();
 }
 

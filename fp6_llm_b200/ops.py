@@ -295,6 +295,17 @@ def quantize_prepack_cuda(weights: torch.Tensor, scales: torch.Tensor, EXPONENT:
     return out
 
 
+def row_scales_cuda(weights: torch.Tensor, top: float) -> torch.Tensor:
+    """fp16 CUDA weights [OC, IC] (contiguous, IC % 8 == 0, 16-byte aligned) -> fp16 [OC]: max|w| of every row divided by
+    `top`, at least 2^-24, in one pass over the weights (C: fp6b200_row_scales; no counterpart in the reference)."""
+    OC, IC = weights.shape
+    out = torch.empty(OC, dtype=torch.float16, device=weights.device)
+    with torch.cuda.device(weights.device):
+        rc = _native.lib().fp6b200_row_scales(_stream_ptr(weights.device), _ptr(weights), _ptr(out), OC, IC, top)
+    _native.check(rc, "fp6b200_row_scales")
+    return out
+
+
 def weight_prepacking_cpu(fp6_tensor: torch.Tensor) -> torch.Tensor:
     """FP6 case of :func:`weight_prepacking_eXmY_cpu` (weight_matrix_prepacking_cpu, fp6_llm/csrc/fp6_linear.cu:211-223)."""
     return weight_prepacking_eXmY_cpu(3, 2, fp6_tensor)

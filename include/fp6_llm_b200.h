@@ -149,6 +149,14 @@ int fp6b200_quantize_prepack(int e_bits, int m_bits, void* stream, const void* w
                              void* packed_dev, size_t M, size_t K);
 
 /*
+ * Row scales for that quantiser: scales[m] = max over k of |weights[m][k]| divided by `top` (the format's largest magnitude;
+ * as a multiplication by its fp32 reciprocal), at least 2^-24, as fp16.  NaN in a row gives NaN.  No counterpart in the
+ * reference.  Needs K % 8 == 0 and weights on a 16-byte boundary.
+ */
+int fp6b200_row_scales(void* stream, const void* weights_fp16_dev, void* scales_dev, size_t M, size_t K, float top);
+
+
+/*
  * Weight prepacking on device buffers (in != out), asynchronous on `stream`.
  * GPU counterpart of weight_matrix_prepacking_fp_eXmY (fp6_llm/csrc/utils/weight_prepacking.h:204-211);
  * the output is bit-identical.  Needs M % 64 == 0 and K % 64 == 0 (:121-122).

@@ -1,0 +1,57 @@
+"""The weight-format kernels at the edges of their units: odd multiples of 64 columns, few rows, unaligned inputs, and every
+kind of value that leaves the quantiser's short path."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import ALL_FORMATS
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("e,m", ALL_FORMATS)
+@pytest.mark.parametrize("rows,cols", [(256, 64), (256, 1088), (512, 576)])
+def test_quantiser_takes_every_weight_like_the_definition(native_lib, e, m, rows, cols):
+    """Bits of quantize_rtn -> pack -> prepack on weights drawn from ALL fp16 patterns (infinities and NaN only in rows of
+    their own), on weights that sit exactly on midpoints, and with zero, negative, subnormal, infinite and NaN scales."""
+    import fp6_llm_b200 as f
+    from fp6_llm_b200.formats import magnitudes, pack_codes, quantize_rtn
+    gen = torch.Generator().manual_seed(rows + cols)
+    w = torch.randint(0, 0x7c00, (rows, cols), generator=gen, dtype=torch.int32)
+    w = (w | (torch.randint(0, 2, (rows, cols), generator=gen, dtype=torch.int32) << 15)).to(torch.uint16).view(torch.float16)
+    scale = (torch.rand(rows, generator=gen) * 2000 + 1e-3).half()
+    scale[5], scale[6], scale[7] = 6e-8, 3e-5, 65504.0
+    # rows of exact ties: midpoint * scale, where the product is an fp16 number
+    mag = magnitudes(e, m)
+    mid = torch.cat([(mag[:-1] + mag[1:]) / 2, mag])
+    for r in range(16, 48):
+        scale[r] = 2.0 ** (r - 36) * (1 + (r % 8) / 8)
+        w[r] = (mid[torch.randint(0, len(mid), (cols,), generator=gen)] * scale[r].float()).half()
+    w[60, ::7], w[60, 3::7], w[61, 5] = float("inf"), float("-inf"), float("-inf")
+    scale[62], scale[63] = -0.5, float("inf")
+    codes = quantize_rtn(w, scale, e, m)
+    got = f.quantize_prepack_cuda(w.cuda(), scale.cuda(), e, m)
+    expect = f.weight_prepacking_eXmY_cpu(e, m, pack_codes(codes, e, m).cuda())
+    assert torch.equal(got, expect)
+    # weights that start on a 4-byte but not on a 16-byte boundary
+    store = torch.empty(rows * cols + 8, dtype=torch.float16, device="cuda")
+    shifted = store[2:2 + rows * cols].view(rows, cols)
+    shifted.copy_(w)
+    assert torch.equal(f.quantize_prepack_cuda(shifted, scale.cuda(), e, m), expect)
+
+
+@pytest.mark.parametrize("cols", [8, 64, 2056, 8192 + 64])
+def test_row_scales_match_the_tensor_expression(native_lib, cols):
+    from fp6_llm_b200 import FPxLinear
+    gen = torch.Generator().manual_seed(cols)
+    w = (torch.randn(37, cols, generator=gen) * 0.02).half()
+    w[3], w[4, -1], w[5, 0], w[6] = 0.0, float("-inf"), float("nan"), 6e-8
+    w[7, cols // 2] = -65504.0
+    for e, m in ALL_FORMATS:
+        from fp6_llm_b200.formats import magnitudes
+        top = float(magnitudes(e, m)[-1])
+        d = w.cuda()
+        expect = (d.float().abs().amax(dim=1) / top).clamp_min(2.0 ** -24).to(torch.float16)
+        got = FPxLinear.row_scales(d, e, m)
+        assert np.array_equal(torch.nan_to_num(got, nan=-1.0).cpu().numpy(), torch.nan_to_num(expect, nan=-1.0).cpu().numpy())
+        assert torch.equal(torch.isnan(got), torch.isnan(expect))
