@@ -7,6 +7,7 @@
 // What is exchanged is already in the byte order of the packed words:
 //   b word = [code(r1, 2t+1) | code(r0, 2t+1) | ...] as below: four codes of the row pair r0 = g + 16k, r1 = r0 + 8.
 #pragma once
+#include <cuda_fp16.h>
 #include <stdint.h>
 
 #include "fpx_layout.h"
@@ -21,6 +22,13 @@ __device__ __forceinline__ void rows_to_quad_words(uint32_t r0_lo, uint32_t r0_h
     b[1] = __byte_perm(r0_lo, r1_lo, 0x3726);
     b[2] = __byte_perm(r0_hi, r1_hi, 0x1504);
     b[3] = __byte_perm(r0_hi, r1_hi, 0x3726);
+}
+// The same for rows whose column 0 is in the HIGHEST byte of `lo` (codes cut from a big-endian stream).
+__device__ __forceinline__ void stream_rows_to_quad_words(uint32_t r0_lo, uint32_t r0_hi, uint32_t r1_lo, uint32_t r1_hi, uint32_t b[4]) {
+    b[0] = __byte_perm(r0_lo, r1_lo, 0x2637);
+    b[1] = __byte_perm(r0_lo, r1_lo, 0x0415);
+    b[2] = __byte_perm(r0_hi, r1_hi, 0x2637);
+    b[3] = __byte_perm(r0_hi, r1_hi, 0x0415);
 }
 __device__ __forceinline__ void quad_words_to_rows(const uint32_t b[4], uint32_t& r0_lo, uint32_t& r0_hi, uint32_t& r1_lo, uint32_t& r1_hi) {
     r0_lo = __byte_perm(b[0], b[1], 0x7531);
@@ -42,6 +50,47 @@ __device__ __forceinline__ void quad_transpose(uint32_t v[4], int lane) {
             if (up) v[i] = got; else v[i | bit] = got;
         }
     }
+}
+
+// The eight codes of a chunk of the unpacked, MSB-first stream, one per byte, column 0 in the highest byte of lo.  v0: the
+// aligned 32-bit word that holds the chunk's first byte, `at`: which of its bytes that is, v1: the next word.  Chunks of 5
+// or 6 bytes that start on a multiple of their length always reach into v1 and never past it, those of 4 bytes never do.
+template <int BW>
+__device__ __forceinline__ void cut_stream_chunk(uint32_t v0, uint32_t v1, uint32_t at, uint32_t& lo, uint32_t& hi) {
+    uint32_t a, b;   // codes 0..3 and 4..7 in the lowest 4 * BW bits; what lies above is masked off below
+    if constexpr (BW == 6) {
+        a = __byte_perm(v0, v1, 0x0012 + 0x0111 * at);
+        b = __byte_perm(v0, v1, 0x0345 + 0x0111 * at);
+    } else if constexpr (BW == 5) {
+        const uint32_t top = __byte_perm(v0, v1, 0x0123 + 0x1111 * at), last = __byte_perm(v0, v1, 0x0004 + at);
+        a = top >> 12;
+        b = (top << 8) | (last & 0xffu);
+    } else {
+        a = __byte_perm(v0, v1, 0x0001);
+        b = __byte_perm(v0, v1, 0x0023);
+    }
+    constexpr uint32_t code = (1u << BW) - 1u, even = code | (code << 16), odd = even << 8;
+    a = ((a << (16 - 2 * BW)) & 0xffff0000u) | (a & 0xffffu);
+    b = ((b << (16 - 2 * BW)) & 0xffff0000u) | (b & 0xffffu);
+    lo = ((a << (8 - BW)) & odd) | (a & even);
+    hi = ((b << (8 - BW)) & odd) | (b & even);
+}
+
+template <int BW>
+__device__ __forceinline__ void read_stream_chunk(const uint32_t* first, uint32_t at, uint32_t& lo, uint32_t& hi) {
+    cut_stream_chunk<BW>(__ldg(first), BW == 4 ? 0u : __ldg(first + 1), at, lo, hi);
+}
+
+// Two fp16 patterns sign | (exponent, mantissa) >> (5 - E) from codes in the upper bytes of both halves, left-aligned there.
+template <int E_BITS>
+__device__ __forceinline__ uint32_t pattern_pair(uint32_t x) {
+    constexpr uint32_t below = (0x7fffu >> (5 - E_BITS)) * 0x00010001u;
+    return (x & 0x80008000u) | ((x >> (5 - E_BITS)) & below);
+}
+// value = code value * scale in fp16: the first product (by 2^bias) is exact, the second rounds once, as in the reference.
+__device__ __forceinline__ uint32_t scaled_pair(uint32_t pattern, __half2 bias, __half2 scale) {
+    const __half2 v = __hmul2(__hmul2(*reinterpret_cast<const __half2*>(&pattern), bias), scale);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 // The packed words of one unit, built from its b words: add(k, b) takes, for the row pair k (rows g + 16k, g + 16k + 8),

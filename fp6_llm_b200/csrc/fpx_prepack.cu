@@ -19,57 +19,41 @@ namespace fpx {
 
 namespace {
 
-constexpr int kPrepackThreads = 256;
-constexpr int kChunkKBlocks = 4;   // a CTA repacks 64 rows x (up to) 256 columns
+// A CTA of the kernels below = 64 rows x kWarps * kSlots units of 32 columns (fpx_codes.cuh), warps on neighbouring units.
+constexpr int kWarps = 8;
+constexpr int kSlots = 2;
 
-// One CTA: stage 64 rows x chunk columns of the unpacked stream in shared memory (coalesced 4-byte
-// reads), then build every output word of that chunk; each word gathers 32/w segments.
+// Packs the unpacked stream.  A lane cuts its chunks (8 codes, bw bytes) out of two aligned words, neighbouring lanes and
+// warps read neighbouring bytes, and the packed words are put together in registers.  HBM-bound: 30 us = 4.1 TB/s
+// on 10240 x 8192 e3m2 codes.  (Gathering every field of every word from shared memory with the closed form of
+// field_source took 154 us.)
 template <int BW>
-__global__ void __launch_bounds__(kPrepackThreads)
-prepack_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32_t M, uint32_t K) {
-    constexpr uint32_t kMaxChunkBytes = kChunkKBlocks * kKBlock * BW / 8;
-    constexpr uint32_t kPitch = kMaxChunkBytes + 4;
-    __shared__ __align__(16) uint8_t tile[kRowsPerBlock * kPitch];
-
-    const uint32_t kblocks = K / kKBlock;
-    const uint32_t chunks_per_row = (kblocks + kChunkKBlocks - 1) / kChunkKBlocks;
-    const uint32_t i = blockIdx.x / chunks_per_row;            // 64-row block
-    const uint32_t kb0 = (blockIdx.x % chunks_per_row) * kChunkKBlocks;
-    const uint32_t nkb = min((uint32_t)kChunkKBlocks, kblocks - kb0);
-    const uint32_t chunk_bytes = nkb * kKBlock * BW / 8;       // multiple of 8
-    const uint32_t col0 = kb0 * kKBlock;
-    const size_t row_bytes = (size_t)K * BW / 8;
-
-    const uint32_t words_per_row = chunk_bytes / 4;
-    for (uint32_t x = threadIdx.x; x < kRowsPerBlock * words_per_row; x += kPrepackThreads) {
-        const uint32_t r = x / words_per_row, wd = x % words_per_row;
-        const uint32_t v = *reinterpret_cast<const uint32_t*>(in + (size_t)(i * kRowsPerBlock + r) * row_bytes +
-                                                              (size_t)col0 * BW / 8 + wd * 4);
-        *reinterpret_cast<uint32_t*>(tile + r * kPitch + wd * 4) = v;
-    }
-    if (threadIdx.x < kRowsPerBlock) tile[threadIdx.x * kPitch + chunk_bytes] = 0;   // read_code may peek one byte past
-    __syncthreads();
-
+__global__ void __launch_bounds__(kWarps * 32)
+prepack_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32_t K, uint32_t ctas_per_row, uint64_t off2,
+               uint64_t off4) {
+    const uint32_t i = blockIdx.x / ctas_per_row;              // 64-row block
+    const uint32_t first_unit = (blockIdx.x - i * ctas_per_row) * kSlots * kWarps;
+    const int lane = threadIdx.x & 31, g = lane >> 2, s = lane & 3;
+    const uint32_t units = K / 32;
+    const size_t row_bytes = (size_t)K * BW / 8;               // a multiple of 8 * BW
+    const uint32_t at = ((uint32_t)s * BW) & 3u;               // a unit starts on a word: 4 * BW bytes per row
+#pragma unroll 1
+    for (int slot = 0; slot < kSlots; slot++) {
+        const uint32_t unit = first_unit + slot * kWarps + (threadIdx.x >> 5);
+        if (unit >= units) return;
+        const uint8_t* src = in + ((size_t)i * kRowsPerBlock + g) * row_bytes + (size_t)unit * (4 * BW) + (s * BW - at);
+        PackedUnit<BW> words;
 #pragma unroll
-    for (int w = 1; w <= 4; w <<= 1) {
-        if (!has_seg(BW, w)) continue;
-        const int shift = seg_shift(BW, w);
-        const uint32_t words_per_tile = 4u * w * 32u;           // uint32 words of one 64x64 tile in this region
-        uint32_t* region = reinterpret_cast<uint32_t*>(out + region_offset(BW, w, M, K));
-        for (uint32_t x = threadIdx.x; x < nkb * words_per_tile; x += kPrepackThreads) {
-            const uint32_t kb = kb0 + x / words_per_tile;
-            const uint32_t in_tile = x % words_per_tile;
-            const int lane = in_tile & 31;
-            const uint64_t word_in_lane = ((uint64_t)i * kblocks + kb) * (4u * w) + (in_tile >> 5);
-            uint32_t word = 0;
-#pragma unroll 8
-            for (int p = 0; p < 32 / w; p++) {
-                const FieldSource s = field_source(w, word_in_lane, lane, p, K);
-                const uint32_t code = read_code(tile + (s.row - i * kRowsPerBlock) * kPitch, s.col - col0, BW);
-                word |= ((code >> shift) & ((1u << w) - 1u)) << (32 - (p + 1) * w);
-            }
-            region[word_in_lane * 32 + lane] = word;
+        for (int k = 0; k < 4; k++) {
+            uint32_t lo[2], hi[2], b[4];
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+                read_stream_chunk<BW>(reinterpret_cast<const uint32_t*>(src + (size_t)(16 * k + 8 * r) * row_bytes), at, lo[r], hi[r]);
+            stream_rows_to_quad_words(lo[0], hi[0], lo[1], hi[1], b);
+            quad_transpose(b, lane);
+            words.add(k, b);
         }
+        words.store(out, off2, off4, (uint64_t)i * (K / 16) + (uint64_t)unit * 2, lane);
     }
 }
 
@@ -90,9 +74,6 @@ prepack_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, uint32
 //   * rounding to the format by cvt for e3m2 and e2m3, by one addition of a power of two otherwise (round_code).
 //   * a lane reads 16 bytes of a row; the packed words are put together in registers (fpx_codes.cuh).
 // Rows whose scale is zero, negative or not finite, and chunks that hold an infinite or NaN weight, take the exact definition.
-constexpr int kQuantWarps = 8;
-constexpr int kQuantSlots = 2;     // 32-column units per warp: one reciprocal per row and 512 columns
-
 // Code of the magnitude and sign in the bits of a finite float: 2^(23 - M) times the binade's unit (at least the subnormals'
 // binade) is added, so that the addition itself rounds to the format's last bit, ties to even.
 template <int E_BITS, int M_BITS>
@@ -147,13 +128,13 @@ __device__ __noinline__ uint2 exact_codes8(uint4 raw, float scale) {
 }
 
 template <int E_BITS, int M_BITS>
-__global__ void __launch_bounds__(kQuantWarps * 32)
+__global__ void __launch_bounds__(kWarps * 32)
 quantize_prepack_kernel(const __half* __restrict__ w, const __half* __restrict__ scales, uint8_t* __restrict__ out,
                         uint32_t K, uint32_t ctas_per_row, uint64_t off2, uint64_t off4, int aligned16) {
     constexpr int BW = 1 + E_BITS + M_BITS;
     __shared__ float row_scale[kRowsPerBlock], row_inv[kRowsPerBlock];   // row_inv 0: the row takes the exact definition
     const uint32_t i = blockIdx.x / ctas_per_row;              // 64-row block
-    const uint32_t first_unit = (blockIdx.x - i * ctas_per_row) * kQuantSlots * kQuantWarps;
+    const uint32_t first_unit = (blockIdx.x - i * ctas_per_row) * kSlots * kWarps;
     const int lane = threadIdx.x & 31, g = lane >> 2, s = lane & 3;
     if (threadIdx.x < kRowsPerBlock) {
         const float sc = __half2float(scales[(size_t)i * kRowsPerBlock + threadIdx.x]);
@@ -163,8 +144,8 @@ quantize_prepack_kernel(const __half* __restrict__ w, const __half* __restrict__
     __syncthreads();
     const uint32_t units = K / 32;
 #pragma unroll 1
-    for (int slot = 0; slot < kQuantSlots; slot++) {
-        const uint32_t unit = first_unit + slot * kQuantWarps + (threadIdx.x >> 5);
+    for (int slot = 0; slot < kSlots; slot++) {
+        const uint32_t unit = first_unit + slot * kWarps + (threadIdx.x >> 5);
         if (unit >= units) return;
         const __half* src = w + ((size_t)i * kRowsPerBlock + g) * K + (size_t)unit * 32 + s * 8;
         uint4 raw[8];
@@ -246,70 +227,99 @@ __global__ void __launch_bounds__(256) row_scales_kernel(const __half* __restric
     }
 }
 
-// Thread = 8 consecutive codes of one row (BW bytes in, 16 bytes out).
+// Unpacked codes -> fp16.  A warp takes 1024 columns of a row, a lane four chunks of 8 codes, 32 chunks apart: neighbouring lanes
+// read neighbouring bytes (two aligned words per chunk) and write neighbouring 16 bytes.  HBM-bound: 42 us = 5.5 TB/s on
+// 10240 x 8192 e3m2 codes (byte loads and a division of the index per chunk took 54 us).
+constexpr uint32_t kDequantChunks = 128;   // chunks per warp
 template <int E_BITS, int M_BITS>
 __global__ void __launch_bounds__(256)
 dequant_unpacked_kernel(const uint8_t* __restrict__ in, const __half* __restrict__ scales, __half* __restrict__ out,
-                        uint32_t M, uint32_t K) {
+                        uint32_t M, uint32_t K, uint32_t warps_per_row, int aligned4) {
     constexpr int BW = 1 + E_BITS + M_BITS;
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // group of 8 codes
-    const size_t groups_per_row = K / 8;
-    if (idx >= (size_t)M * groups_per_row) return;
-    const size_t row = idx / groups_per_row;
-    const uint8_t* src = in + idx * BW;
-    uint8_t bytes[BW + 1];
+    const uint32_t id = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const uint32_t row = id / warps_per_row;
+    if (row >= M) return;
+    const uint32_t chunks = K / 8, c0 = (id - row * warps_per_row) * kDequantChunks + lane;
+    const __half2 bias = __half2half2(__ushort_as_half(bias_half_bits(E_BITS)));
+    const __half2 scale = __half2half2(scales[row]);
+    const uint8_t* src = in + (size_t)row * chunks * BW;       // a row starts on a word: chunks is a multiple of 8
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * K);
+    uint32_t lo[4], hi[4];
 #pragma unroll
-    for (int b = 0; b < BW; b++) bytes[b] = src[b];
-    bytes[BW] = 0;
-    const float s = __half2float(scales[row]);
-    const float bias = (float)(1u << (16 - (1 << (E_BITS - 1))));
-    __align__(16) __half vals[8];
+    for (int u = 0; u < 4; u++) {
+        const uint32_t c = c0 + 32 * u;
+        lo[u] = hi[u] = 0u;
+        if (c >= chunks) continue;
+        const uint32_t byte = c * BW;
+        if (aligned4) {
+            read_stream_chunk<BW>(reinterpret_cast<const uint32_t*>(src + (byte & ~3u)), byte & 3u, lo[u], hi[u]);
+        } else {   // a stream that starts between two words
+            uint32_t v[2] = {0u, 0u};
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        const uint32_t code = read_code(bytes, c, BW);
-        const uint32_t left = code << (16 - BW);   // code left-aligned in 16 bits
-        const uint16_t h = (uint16_t)((left & 0x8000u) | ((left & 0x7fffu) >> (5 - E_BITS)));
-        vals[c] = __float2half_rn(__half2float(__ushort_as_half(h)) * bias * s);
+            for (int b = 0; b < BW; b++) v[b >> 2] |= (uint32_t)src[byte + b] << (8 * (b & 3));
+            cut_stream_chunk<BW>(v[0], v[1], 0u, lo[u], hi[u]);
+        }
     }
-    *reinterpret_cast<uint4*>(out + idx * 8) = *reinterpret_cast<const uint4*>(vals);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const uint32_t c = c0 + 32 * u;
+        if (c >= chunks) break;
+        const uint32_t l = lo[u] << (8 - BW), h = hi[u] << (8 - BW);   // left-aligned in every byte; columns from the top byte down
+        uint4 v;
+        v.x = scaled_pair(pattern_pair<E_BITS>(__byte_perm(l, 0u, 0x2434)), bias, scale);
+        v.y = scaled_pair(pattern_pair<E_BITS>(__byte_perm(l, 0u, 0x0414)), bias, scale);
+        v.z = scaled_pair(pattern_pair<E_BITS>(__byte_perm(h, 0u, 0x2434)), bias, scale);
+        v.w = scaled_pair(pattern_pair<E_BITS>(__byte_perm(h, 0u, 0x0414)), bias, scale);
+        dst[c] = v;
+    }
 }
 
-// Warp = 32 rows x 64 columns, the unit one unpack warp of the GEMM handles per pipeline stage.
+// Prepacked codes -> fp16: the way of the packers backwards, so that a lane stores 16 bytes of a row.  HBM-bound: 36 us =
+// 6.4 TB/s on 10240 x 8192 e3m2 codes (storing the register pairs of the GEMM's unpack, 4 bytes each, took 70 us).
 template <int E_BITS, int M_BITS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kWarps * 32)
 dequant_packed_kernel(const uint8_t* __restrict__ packed, const __half* __restrict__ scales, __half* __restrict__ out,
-                      uint32_t M, uint32_t K) {
+                      uint32_t K, uint32_t ctas_per_row, uint64_t off2, uint64_t off4, int aligned16) {
     constexpr int BW = 1 + E_BITS + M_BITS;
-    const uint32_t kblocks = K / kKBlock;
-    const uint32_t unit = blockIdx.x * 4 + (threadIdx.x >> 5);     // (64-row block, k-block, half)
-    if (unit >= (M / kRowsPerBlock) * kblocks * 2) return;
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int h = unit & 1;
-    const uint32_t kb = (unit >> 1) % kblocks, i = (unit >> 1) / kblocks;
-    const uint64_t tile = (uint64_t)i * kblocks + kb;
-    const uint32_t* r1 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 1, M, K) + tile * tile_bytes(1));
-    const uint32_t* r2 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 2, M, K) + tile * tile_bytes(2));
-    const uint32_t* r4 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 4, M, K) + tile * tile_bytes(4));
-    const __half bias_h = __ushort_as_half(bias_half_bits(E_BITS));
-    const uint32_t row_base = i * kRowsPerBlock + 32 * h;
+    __shared__ __half row_scale[kRowsPerBlock];
+    const uint32_t i = blockIdx.x / ctas_per_row;              // 64-row block
+    const uint32_t first_unit = (blockIdx.x - i * ctas_per_row) * kSlots * kWarps;
+    const int lane = threadIdx.x & 31, g = lane >> 2, s = lane & 3;
+    if (threadIdx.x < kRowsPerBlock) row_scale[threadIdx.x] = scales[(size_t)i * kRowsPerBlock + threadIdx.x];
+    __syncthreads();
+    const __half2 bias = __half2half2(__ushort_as_half(bias_half_bits(E_BITS)));
+    const uint32_t units = K / 32;
+#pragma unroll 1
+    for (int slot = 0; slot < kSlots; slot++) {
+        const uint32_t unit = first_unit + slot * kWarps + (threadIdx.x >> 5);
+        if (unit >= units) return;
+        PackedUnit<BW> words;
+        words.load(packed, off2, off4, (uint64_t)i * (K / 16) + (uint64_t)unit * 2, lane);
+        __half* dst = out + ((size_t)i * kRowsPerBlock + g) * K + (size_t)unit * 32 + s * 8;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const uint32_t w4a = r4[(j * 4 + 2 * h + 0) * 32 + lane], w4b = r4[(j * 4 + 2 * h + 1) * 32 + lane];
-        const uint32_t w2 = has_seg(BW, 2) ? r2[(j * 2 + h) * 32 + lane] : 0u;
-        const uint32_t w1 = has_seg(BW, 1) ? r1[j * 32 + lane] : 0u;
-        uint32_t pat[8];
-        unpack16_any<E_BITS, M_BITS>(w4a, w4b, w2, w1, h, pat);
+        for (int k = 0; k < 4; k++) {
+            uint32_t b[4], lo[2], hi[2];
+            words.take(k, b);
+            quad_transpose(b, lane);
+            quad_words_to_rows(b, lo[0], hi[0], lo[1], hi[1]);
 #pragma unroll
-        for (int kk = 0; kk < 2; kk++)
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const uint32_t row = row_base + 16 * kk + 8 * (a & 1) + g;
-                const uint32_t col = kb * kKBlock + 16 * j + 8 * (a >> 1) + 2 * t;
-                const __half s = scales[row];
-                __half2 v = *reinterpret_cast<__half2*>(&pat[4 * kk + a]);
-                v = __hmul2(__hmul2(v, __half2half2(bias_h)), __half2half2(s));   // first product is exact
-                *reinterpret_cast<__half2*>(out + (size_t)row * K + col) = v;
+            for (int r = 0; r < 2; r++) {
+                const __half2 scale = __half2half2(row_scale[16 * k + 8 * r + g]);
+                const uint32_t l = lo[r] << (8 - BW), h = hi[r] << (8 - BW);
+                uint4 v;
+                v.x = scaled_pair(pattern_pair<E_BITS>(__byte_perm(l, 0u, 0x1404)), bias, scale);
+                v.y = scaled_pair(pattern_pair<E_BITS>(__byte_perm(l, 0u, 0x3424)), bias, scale);
+                v.z = scaled_pair(pattern_pair<E_BITS>(__byte_perm(h, 0u, 0x1404)), bias, scale);
+                v.w = scaled_pair(pattern_pair<E_BITS>(__byte_perm(h, 0u, 0x3424)), bias, scale);
+                __half* p = dst + (size_t)(16 * k + 8 * r) * K;
+                if (aligned16) {
+                    *reinterpret_cast<uint4*>(p) = v;
+                } else {
+                    uint32_t* p4 = reinterpret_cast<uint32_t*>(p);
+                    p4[0] = v.x; p4[1] = v.y; p4[2] = v.z; p4[3] = v.w;
+                }
             }
+        }
     }
 }
 
@@ -321,20 +331,32 @@ bool shape_ok(int e_bits, int m_bits, size_t M, size_t K) {
 
 }  // namespace
 
+namespace {
+// CTAs of a kernel that takes 64 rows x kWarps * kSlots units per CTA: per row of blocks, and in all (0: too many)
+size_t unit_ctas(size_t M, size_t K, uint32_t* per_row) {
+    const uint32_t per_cta = kWarps * kSlots;
+    *per_row = ((uint32_t)(K / 32) + per_cta - 1) / per_cta;
+    const size_t ctas = (M / kRowsPerBlock) * *per_row;
+    return ctas <= 0x7fffffffull ? ctas : 0;
+}
+}  // namespace
+
 cudaError_t launch_prepack(int e_bits, int m_bits, cudaStream_t stream, const void* unpacked, void* packed, size_t M,
                            size_t K) {
     if (!shape_ok(e_bits, m_bits, M, K) || !unpacked || !packed || unpacked == packed) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(unpacked) & 3) || (reinterpret_cast<uintptr_t>(packed) & 3))
         return cudaErrorMisalignedAddress;
-    const size_t kblocks = K / kKBlock;
-    const size_t blocks = (M / kRowsPerBlock) * ((kblocks + kChunkKBlocks - 1) / kChunkKBlocks);
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    uint32_t per_row = 0;
+    const size_t ctas = unit_ctas(M, K, &per_row);
+    if (ctas == 0) return cudaErrorInvalidValue;
     const uint8_t* in = static_cast<const uint8_t*>(unpacked);
     uint8_t* out = static_cast<uint8_t*>(packed);
-    switch (1 + e_bits + m_bits) {
-        case 4:  prepack_kernel<4><<<(unsigned)blocks, kPrepackThreads, 0, stream>>>(in, out, (uint32_t)M, (uint32_t)K); break;
-        case 5:  prepack_kernel<5><<<(unsigned)blocks, kPrepackThreads, 0, stream>>>(in, out, (uint32_t)M, (uint32_t)K); break;
-        default: prepack_kernel<6><<<(unsigned)blocks, kPrepackThreads, 0, stream>>>(in, out, (uint32_t)M, (uint32_t)K); break;
+    const int bw = bit_width(e_bits, m_bits);
+    const uint64_t off2 = region_offset(bw, 2, M, K), off4 = region_offset(bw, 4, M, K);
+    switch (bw) {
+        case 4:  prepack_kernel<4><<<(unsigned)ctas, kWarps * 32, 0, stream>>>(in, out, (uint32_t)K, per_row, off2, off4); break;
+        case 5:  prepack_kernel<5><<<(unsigned)ctas, kWarps * 32, 0, stream>>>(in, out, (uint32_t)K, per_row, off2, off4); break;
+        default: prepack_kernel<6><<<(unsigned)ctas, kWarps * 32, 0, stream>>>(in, out, (uint32_t)K, per_row, off2, off4); break;
     }
     return cudaGetLastError();
 }
@@ -347,12 +369,11 @@ cudaError_t launch_quantize_prepack(int e_bits, int m_bits, cudaStream_t stream,
     uint8_t* out = static_cast<uint8_t*>(packed);
     const int bw = bit_width(e_bits, m_bits);
     const uint64_t off2 = region_offset(bw, 2, M, K), off4 = region_offset(bw, 4, M, K);
-    const uint32_t units = (uint32_t)(K / 32), per_cta = kQuantWarps * kQuantSlots;
     const int aligned16 = (reinterpret_cast<uintptr_t>(weights) & 15) == 0;
-    const uint32_t ctas_per_row = (units + per_cta - 1) / per_cta;
-    const size_t blocks = (M / kRowsPerBlock) * ctas_per_row;
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-    FPX_DISPATCH_FORMAT(e_bits, m_bits, (quantize_prepack_kernel<kE, kM><<<(unsigned)blocks, kQuantWarps * 32, 0, stream>>>(weights, scales, out, (uint32_t)K, ctas_per_row, off2, off4, aligned16)));
+    uint32_t per_row = 0;
+    const size_t ctas = unit_ctas(M, K, &per_row);
+    if (ctas == 0) return cudaErrorInvalidValue;
+    FPX_DISPATCH_FORMAT(e_bits, m_bits, (quantize_prepack_kernel<kE, kM><<<(unsigned)ctas, kWarps * 32, 0, stream>>>(weights, scales, out, (uint32_t)K, per_row, off2, off4, aligned16)));
     return cudaGetLastError();
 }
 
@@ -368,11 +389,12 @@ cudaError_t launch_dequant_unpacked(int e_bits, int m_bits, cudaStream_t stream,
                                     const __half* scales, __half* out, size_t M, size_t K) {
     if (!shape_ok(e_bits, m_bits, M, K) || !unpacked || !scales || !out) return cudaErrorInvalidValue;
     if (reinterpret_cast<uintptr_t>(out) & 15) return cudaErrorMisalignedAddress;
-    const size_t groups = M * (K / 8);
-    const size_t blocks = (groups + 255) / 256;
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    const uint32_t warps_per_row = ((uint32_t)(K / 8) + kDequantChunks - 1) / kDequantChunks;
+    const size_t warps = M * warps_per_row;
+    if (warps > 0xffffffffull - 8) return cudaErrorInvalidValue;
+    const unsigned ctas = (unsigned)((warps + 7) / 8);
     const uint8_t* in = static_cast<const uint8_t*>(unpacked);
-    FPX_DISPATCH_FORMAT(e_bits, m_bits, (dequant_unpacked_kernel<kE, kM><<<(unsigned)blocks, 256, 0, stream>>>(in, scales, out, (uint32_t)M, (uint32_t)K)));
+    FPX_DISPATCH_FORMAT(e_bits, m_bits, (dequant_unpacked_kernel<kE, kM><<<ctas, 256, 0, stream>>>(in, scales, out, (uint32_t)M, (uint32_t)K, warps_per_row, (reinterpret_cast<uintptr_t>(unpacked) & 3) == 0)));
     return cudaGetLastError();
 }
 
@@ -381,11 +403,14 @@ cudaError_t launch_dequant_packed(int e_bits, int m_bits, cudaStream_t stream, c
     if (!shape_ok(e_bits, m_bits, M, K) || !packed || !scales || !out) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(packed) & 15) || (reinterpret_cast<uintptr_t>(out) & 3))
         return cudaErrorMisalignedAddress;
-    const size_t units = (M / kRowsPerBlock) * (K / kKBlock) * 2;
-    const size_t blocks = (units + 3) / 4;
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    uint32_t per_row = 0;
+    const size_t ctas = unit_ctas(M, K, &per_row);
+    if (ctas == 0) return cudaErrorInvalidValue;
     const uint8_t* in = static_cast<const uint8_t*>(packed);
-    FPX_DISPATCH_FORMAT(e_bits, m_bits, (dequant_packed_kernel<kE, kM><<<(unsigned)blocks, 128, 0, stream>>>(in, scales, out, (uint32_t)M, (uint32_t)K)));
+    const int bw = bit_width(e_bits, m_bits);
+    const uint64_t off2 = region_offset(bw, 2, M, K), off4 = region_offset(bw, 4, M, K);
+    const int aligned16 = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    FPX_DISPATCH_FORMAT(e_bits, m_bits, (dequant_packed_kernel<kE, kM><<<(unsigned)ctas, kWarps * 32, 0, stream>>>(in, scales, out, (uint32_t)K, per_row, off2, off4, aligned16)));
     return cudaGetLastError();
 }
 

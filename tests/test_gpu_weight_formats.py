@@ -55,3 +55,36 @@ def test_row_scales_match_the_tensor_expression(native_lib, cols):
         got = FPxLinear.row_scales(d, e, m)
         assert np.array_equal(torch.nan_to_num(got, nan=-1.0).cpu().numpy(), torch.nan_to_num(expect, nan=-1.0).cpu().numpy())
         assert torch.equal(torch.isnan(got), torch.isnan(expect))
+
+
+@pytest.mark.parametrize("e,m", ALL_FORMATS)
+@pytest.mark.parametrize("rows,cols", [(64, 64), (128, 576), (192, 1088)])
+def test_packer_and_dequantisers_at_unit_edges(native_lib, oracle_mod, e, m, rows, cols):
+    """Columns that leave the last CTA, warp and lane group partly empty; every result bit-exact against the oracle."""
+    import ctypes
+    import fp6_llm_b200 as f
+    from helpers import random_unpacked
+    rng = np.random.default_rng(rows + cols + 8 * e + m)
+    w = random_unpacked(rng, rows, cols, e, m)
+    s = (rng.random(rows) * 0.01 + 1e-3).astype(np.float16)
+    s[0], s[1], s[2] = 6e-8, 65504.0, np.inf
+    d, sd = torch.from_numpy(w).cuda(), torch.from_numpy(s).cuda()
+    packed = torch.empty_like(d)
+    assert native_lib.fp6b200_prepack(e, m, None, d.data_ptr(), packed.data_ptr(), rows, cols) == 0   # 64-row granularity
+    torch.cuda.synchronize()
+    assert np.array_equal(packed.cpu().numpy(), oracle_mod.prepack(w, e, m))
+    want = oracle_mod.dequant(w, s, e, m)
+    same = lambda t: np.array_equal(t.cpu().numpy(), want, equal_nan=True)   # noqa: E731
+    assert same(f.weight_dequant_eXmY_cpu(e, m, d, sd))
+    assert same(f.dequant_packed_cuda(e, m, packed, sd))
+    # a code stream that starts on an odd byte, and an fp16 result that starts on a 4-byte boundary
+    raw = torch.empty(w.nbytes + 16, dtype=torch.uint8, device="cuda")
+    raw[3:3 + w.nbytes] = d.view(torch.uint8).reshape(-1)
+    out = torch.empty(rows, cols, dtype=torch.float16, device="cuda")
+    assert native_lib.fp6b200_dequant(e, m, None, ctypes.c_void_p(raw.data_ptr() + 3), sd.data_ptr(), out.data_ptr(), rows, cols) == 0
+    torch.cuda.synchronize()
+    assert same(out)
+    store = torch.empty(rows * cols + 8, dtype=torch.float16, device="cuda")
+    assert native_lib.fp6b200_dequant_packed(e, m, None, packed.data_ptr(), sd.data_ptr(), ctypes.c_void_p(store.data_ptr() + 4), rows, cols) == 0
+    torch.cuda.synchronize()
+    assert same(store[2:2 + rows * cols].view(rows, cols))
