@@ -76,6 +76,12 @@ __device__ __forceinline__ void cut_stream_chunk(uint32_t v0, uint32_t v1, uint3
     hi = ((b << (8 - BW)) & odd) | (b & even);
 }
 
+// Four six-bit codes, one per byte, column 0 in the lowest -> 24 bits, code i at bits 6i .. 6i + 5.
+__device__ __forceinline__ uint32_t join_codes6(uint32_t c) {
+    const uint32_t two = (c & 0x003f003fu) | ((c >> 2) & 0x0fc00fc0u);
+    return (two & 0xfffu) | ((two >> 4) & 0xfff000u);
+}
+
 template <int BW>
 __device__ __forceinline__ void read_stream_chunk(const uint32_t* first, uint32_t at, uint32_t& lo, uint32_t& hi) {
     cut_stream_chunk<BW>(__ldg(first), BW == 4 ? 0u : __ldg(first + 1), at, lo, hi);

@@ -93,6 +93,10 @@ size_t gemm_auto_workspace_bytes(size_t N);
 
 // The tensor cores' own six-bit inputs (fpx_native.cu): e3m2 and e2m3 weights re-laid into 128 x 128 tiles that a tensor
 // copy expands in flight, activations split into four exact e5m2 planes; batches of up to native_max_tokens() tokens.
+constexpr int kNatTileM = 128;                  // rows of a weight tile = M of the MMA
+constexpr int kNatTileK = 128;                  // K of a weight tile = one 128-byte swizzle row of shared memory
+constexpr int kNatRowBytes = kNatTileK * 6 / 8;           // 96 bytes of HBM per tile row
+constexpr int kNatTileBytes = kNatTileM * kNatRowBytes;   // 12 KB of HBM per tile
 bool native_format(int e_bits, int m_bits);
 int native_max_tokens();
 size_t native_weight_bytes(size_t M, size_t K);

@@ -45,10 +45,6 @@ namespace fpx {
 
 namespace {
 
-constexpr int kNatTileM = 128;                  // rows of a weight tile = M of the MMA
-constexpr int kNatTileK = 128;                  // K of a weight tile = one 128-byte swizzle row of shared memory
-constexpr int kNatRowBytes = kNatTileK * 6 / 8;        // 96 bytes of HBM per tile row
-constexpr int kNatTileBytes = kNatTileM * kNatRowBytes;   // 12 KB of HBM per tile
 constexpr uint32_t kNatTileSmem = kNatTileM * 128;     // 16 KB of shared memory per tile (16 codes -> 16 bytes)
 constexpr int kPieces = 4;
 // Optional milestones of every CTA (build with -DFPX_PROFILE): global-timer stamps read back with
@@ -554,77 +550,6 @@ __global__ void __launch_bounds__(256) split_activations_kernel(const __half* __
         *reinterpret_cast<uint2*>(planes + (size_t)(pc * tokens + n) * kpad + k0) = make_uint2(out[pc][0], out[pc][1]);
 }
 
-// ------------------------------------------------------------------------------------------------
-// Reference-packed weights -> native tiles.  A warp takes the 32 rows x 64 columns one unpack warp of the fp16 path
-// handles (same words, same unpack sequence), recovers the codes from the fp16 patterns (widened to six bits), gathers
-// them in shared memory and writes every 16 codes of a row as 12 bytes, code i at bits 6 i .. 6 i + 5.
-template <int E_BITS, int M_BITS>
-__global__ void __launch_bounds__(128) native_repack_kernel(const uint8_t* __restrict__ packed, uint8_t* __restrict__ native,
-                                                            uint32_t M, uint32_t K, uint32_t ktiles) {
-    constexpr int BW = 1 + E_BITS + M_BITS;
-    static_assert(BW <= 6, "codes of at most six bits");
-    __shared__ uint8_t codes[4][32][64 + 4];
-    const uint32_t kblocks = K / kKBlock;
-    const int w = threadIdx.x >> 5;
-    const uint32_t unit = blockIdx.x * 4 + w;     // (64-row block, k-block, half)
-    const bool live = unit < (M / kRowsPerBlock) * kblocks * 2;
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    const int h = unit & 1;
-    const uint32_t kb = (unit >> 1) % kblocks, i = (unit >> 1) / kblocks;
-    if (live) {
-        const uint64_t tile = (uint64_t)i * kblocks + kb;
-        const uint32_t* r1 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 1, M, K) + tile * tile_bytes(1));
-        const uint32_t* r2 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 2, M, K) + tile * tile_bytes(2));
-        const uint32_t* r4 = reinterpret_cast<const uint32_t*>(packed + region_offset(BW, 4, M, K) + tile * tile_bytes(4));
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const uint32_t w4a = r4[(j * 4 + 2 * h + 0) * 32 + lane], w4b = r4[(j * 4 + 2 * h + 1) * 32 + lane];
-            const uint32_t w2 = has_seg(BW, 2) ? r2[(j * 2 + h) * 32 + lane] : 0u;
-            const uint32_t w1 = has_seg(BW, 1) ? r1[j * 32 + lane] : 0u;
-            uint32_t pat[8];
-            unpack16_any<E_BITS, M_BITS>(w4a, w4b, w2, w1, h, pat);
-#pragma unroll
-            for (int kk = 0; kk < 2; kk++)
-#pragma unroll
-                for (int a = 0; a < 4; a++) {
-                    const int row = 16 * kk + 8 * (a & 1) + g;
-                    const int col = 16 * j + 8 * (a >> 1) + 2 * t;
-                    const uint32_t v = pat[4 * kk + a];
-                    // pattern = sign | (exponent, mantissa) >> (5 - E): exponent and mantissa are the E + M bits from bit
-                    // 10 - M up.  The six-bit code of the same value in the hardware format with E exponent bits (e3m2
-                    // or e2m3) has the same fields with the mantissa extended by zeros: shift left by 5 - E - M.
-                    constexpr int sh = 10 - M_BITS, ext = 5 - E_BITS - M_BITS;
-                    constexpr uint32_t mask = (1u << (E_BITS + M_BITS)) - 1u;
-                    codes[w][row][col] = (uint8_t)(((v >> 10) & 0x20u) | (((v >> sh) & mask) << ext));
-                    codes[w][row][col + 1] = (uint8_t)(((v >> 26) & 0x20u) | (((v >> (16 + sh)) & mask) << ext));
-                }
-        }
-    }
-    __syncwarp();
-    if (live) {
-        // 32 rows x 4 groups of 16 codes: four groups per lane
-#pragma unroll
-        for (int s = 0; s < 4; s++) {
-            const int grp = s * 32 + lane;
-            const int row = grp >> 2, c0 = (grp & 3) * 16;
-            uint32_t words[3] = {0u, 0u, 0u};
-#pragma unroll
-            for (int c = 0; c < 16; c++) {
-                const uint32_t code = codes[w][row][c0 + c];
-                const int bit = 6 * c;
-                words[bit >> 5] |= code << (bit & 31);
-                if ((bit & 31) > 26) words[(bit >> 5) + 1] |= code >> (32 - (bit & 31));
-            }
-            const uint32_t grow = i * kRowsPerBlock + 32 * h + row;       // global row
-            const uint32_t gcol = kb * kKBlock + c0;                      // global column
-            const size_t tile = (size_t)(grow / kNatTileM) * ktiles + gcol / kNatTileK;
-            uint8_t* dst = native + (tile * kNatTileM + grow % kNatTileM) * kNatRowBytes + (gcol % kNatTileK) * 6 / 8;
-            uint32_t* d32 = reinterpret_cast<uint32_t*>(dst);
-            d32[0] = words[0]; d32[1] = words[1]; d32[2] = words[2];
-        }
-    }
-}
-
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -685,24 +610,6 @@ static size_t native_planes_bytes(size_t N, size_t K) {
 size_t native_workspace_bytes(size_t N, size_t K) {
     const size_t ctas = device_sm_count() < 256 ? device_sm_count() : 256;
     return native_planes_bytes(N, K) + 2 * ctas * kNatTileM * (native_n_tile(N) / kPieces) * sizeof(float);
-}
-
-cudaError_t launch_native_repack(int e_bits, int m_bits, cudaStream_t stream, const void* packed, void* native, size_t M, size_t K) {
-    if (!native_format(e_bits, m_bits) || !packed || !native || packed == native) return cudaErrorInvalidValue;
-    if (M == 0 || M % 256 != 0 || K == 0 || K % 64 != 0 || M > 0x7fffffffull || K > 0x7fffffffull) return cudaErrorInvalidValue;
-    if ((reinterpret_cast<uintptr_t>(packed) & 3) || (reinterpret_cast<uintptr_t>(native) & 15)) return cudaErrorMisalignedAddress;
-    const size_t ktiles = native_ktiles(K);
-    if (K % kNatTileK != 0) {   // the last K tile is half empty: code 0 is +0
-        cudaError_t err = cudaMemsetAsync(native, 0, native_weight_bytes(M, K), stream);
-        if (err != cudaSuccess) return err;
-    }
-    const size_t units = (M / kRowsPerBlock) * (K / kKBlock) * 2;
-    const size_t blocks = (units + 3) / 4;
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-    const uint8_t* in = static_cast<const uint8_t*>(packed);
-    uint8_t* out = static_cast<uint8_t*>(native);
-    FPX_DISPATCH_FORMAT(e_bits, m_bits, (native_repack_kernel<kE, kM><<<(unsigned)blocks, 128, 0, stream>>>(in, out, (uint32_t)M, (uint32_t)K, (uint32_t)ktiles)));
-    return cudaGetLastError();
 }
 
 cudaError_t launch_native_gemm(int e_bits, int m_bits, cudaStream_t stream, const void* weight_native, const __half* scales,
