@@ -16,7 +16,7 @@ _CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libfp6_b200.so")
 SOURCES = ("fpx_gemm.cu", "fpx_native.cu", "fpx_prepack.cu", "c_api.cu", "c_api_noalloc.cu")
-HEADERS = ("fpx_codes.cuh", "fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
+HEADERS = ("fpx_codes.cuh", "fpx_epilogue.cuh", "fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--threads", "4",
               "-Xcompiler", "-fPIC", "-shared"]

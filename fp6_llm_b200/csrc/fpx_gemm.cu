@@ -48,6 +48,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fpx_epilogue.cuh"
 #include "fpx_internal.h"
 #include "fpx_layout.h"
 #include "ptx_sm100.cuh"
@@ -218,9 +219,6 @@ __device__ unsigned long long g_trace[12][64];
 #endif
 
 constexpr uint32_t kMaxGrid = 256;   // CTAs the fix-up kernel's slot list can hold
-
-// silu(gate) * up in fp32
-__device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }
 
 struct Params {
     const uint8_t* weight;
@@ -581,29 +579,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                 if (seg.out_kind == kOutDirect) {
 #pragma unroll
                     for (int u = 0; u < CH; u++) f[u] = f[u] * row_scale + row_bias;
-                    if (p.activation == kActSiluMul) {
-                        // rows 2c (gate) and 2c+1 (up) sit in neighbouring lanes: the even lane computes and stores channel c
-#pragma unroll
-                        for (int u = 0; u < CH; u++) {
-                            const float up = __shfl_xor_sync(0xffffffffu, f[u], 1);
-                            f[u] = silu_mul(f[u], up);
-                        }
-                        if ((lane & 1) == 0) {
-                            __half* dst = p.out.ptr[0] + (size_t)n0 * p.out.ld + p.out.row0 + (row >> 1);
-#pragma unroll
-                            for (int u = 0; u < CH; u++)
-                                if (n0 + u < p.N) dst[(size_t)u * p.out.ld] = __float2half_rn(f[u]);
-                        }
-                    } else {
-                        const size_t first = (size_t)n0 * p.out.ld + p.out.row0 + row;
-#pragma unroll 1
-                        for (uint32_t r = 0; r < p.out.count; r++) {   // one target, or the buffer of every rank
-                            __half* dst = p.out.ptr[r] + first;
-#pragma unroll
-                            for (int u = 0; u < CH; u++)
-                                if (n0 + u < p.N) dst[(size_t)u * p.out.ld] = __float2half_rn(f[u]);
-                        }
-                    }
+                    store_columns(p.out, (int)p.activation, f, n0, p.N, row, lane);
                 } else if (seg.out_kind == kOutSplitPartial) {
                     float* dst = p.workspace + ((size_t)seg.out_index * p.N + n0) * p.M + row;
 #pragma unroll

@@ -37,6 +37,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fpx_epilogue.cuh"
 #include "fpx_internal.h"
 #include "fpx_layout.h"
 #include "ptx_sm100.cuh"
@@ -112,8 +113,6 @@ struct NatParams {
     WorkPlan plan;
     int* status;
 };
-
-__device__ __forceinline__ float silu_mul_f(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }
 
 template <int N_TILE>
 __global__ void __launch_bounds__(NatCfg<N_TILE>::threads, 1)
@@ -452,29 +451,7 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
                 if (seg.out_kind == kOutDirect) {
 #pragma unroll
                     for (int u = 0; u < CH; u++) f[u] = f[u] * row_scale + row_bias;
-                    if (p.activation == kActSiluMul) {
-                        // rows 2c (gate) and 2c+1 (up) sit in neighbouring lanes: the even lane stores channel c
-#pragma unroll
-                        for (int u = 0; u < CH; u++) {
-                            const float up = __shfl_xor_sync(0xffffffffu, f[u], 1);
-                            f[u] = silu_mul_f(f[u], up);
-                        }
-                        if ((lane & 1) == 0) {
-                            __half* dst = p.out.ptr[0] + (size_t)n0 * p.out.ld + p.out.row0 + (row >> 1);
-#pragma unroll
-                            for (int u = 0; u < CH; u++)
-                                if (n0 + u < p.N) dst[(size_t)u * p.out.ld] = __float2half_rn(f[u]);
-                        }
-                    } else {
-                        const size_t first = (size_t)n0 * p.out.ld + p.out.row0 + row;
-#pragma unroll 1
-                        for (uint32_t r = 0; r < p.out.count; r++) {   // one target, or the buffer of every rank
-                            __half* dst = p.out.ptr[r] + first;
-#pragma unroll
-                            for (int u = 0; u < CH; u++)
-                                if (n0 + u < p.N) dst[(size_t)u * p.out.ld] = __float2half_rn(f[u]);
-                        }
-                    }
+                    store_columns(p.out, (int)p.activation, f, n0, p.N, row, lane);
                 } else {   // part of a tile: fp32, scaled, into this CTA's slot [tokens][128]
                     float* dst = p.workspace + ((size_t)seg.out_index * T + t0) * kNatTileM + row_in_tile;
 #pragma unroll

@@ -58,6 +58,38 @@ def test_silu_mul(oracle_mod, oc, ic, bs, split_k, with_bias):
     _close(oracle_mod, y, truth)
 
 
+@pytest.mark.parametrize("bs", [1, 2, 3, 5, 7, 9, 13, 15, 17, 31, 63, 77, 131])
+@pytest.mark.parametrize("silu", [False, True])
+def test_store_tails(oracle_mod, bs, silu):
+    """The lanes of a warp exchange rows and store four of them for every second, fourth or eighth column: token counts that
+    end anywhere inside those groups, tiles stored by the GEMM itself (split 1, and the tile layout's whole tiles)."""
+    import fp6_llm_b200 as f
+    oc, ic = 512, 128
+    packed, s, x, bias, plain = _problem(oracle_mod, 3, 2, oc, ic, bs, seed=bs)
+    pre = plain + bias.float().numpy()[None, :]
+    truth = pre[:, 0::2] / (1.0 + np.exp(-pre[:, 0::2])) * pre[:, 1::2] if silu else pre
+    act = f.ACT_SILU_MUL if silu else f.ACT_NONE
+    _close(oracle_mod, f.linear_forward_ex(3, 2, x, packed, s, 1, bias.cuda(), act), truth)
+    if f.native_supported(3, 2, oc, ic, bs):
+        _close(oracle_mod, f.linear_forward_native(3, 2, x, f.native_repack(3, 2, packed), s, bias.cuda(), act), truth)
+
+
+def test_silu_mul_extremes():
+    """silu at the ends of fp32: exp(-gate) overflows, exp(-gate) just below overflow, gate far positive, both signs of up."""
+    import fp6_llm_b200 as f
+    oc, ic, bs = 256, 64, 4
+    gates = torch.tensor([-60000.0, -89.0, -88.0, -87.5, -20.0, 0.0, 20.0, 60000.0]).half()
+    bias = torch.zeros(oc).half()
+    bias[0::2] = gates.repeat(oc // 16)
+    bias[1::2] = torch.tensor([3.0, -3.0]).half().repeat(oc // 4)
+    x = torch.zeros(bs, ic, dtype=torch.float16, device="cuda")
+    packed = torch.zeros(oc, ic * 6 // 32, dtype=torch.int32, device="cuda")
+    y = f.linear_forward_ex(3, 2, x, packed, torch.ones(oc, dtype=torch.float16, device="cuda"), 1, bias.cuda(), f.ACT_SILU_MUL)
+    g, u = bias[0::2].double(), bias[1::2].double()
+    truth = torch.nn.functional.silu(g) * u
+    assert torch.allclose(y.double().cpu(), truth.half().double().expand(bs, -1), rtol=1e-3, atol=6e-8)
+
+
 def test_gate_up_module_matches_two_linears():
     """FPxGateUpLinear.from_linears: interleaves, quantises and packs two torch layers; its output equals silu(gate) * up
     computed in fp32 from the dequantised weights, and FPxLinear adds its bias inside the kernel."""
