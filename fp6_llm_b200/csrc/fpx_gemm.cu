@@ -231,6 +231,8 @@ struct Params {
     uint32_t activation;        // kActNone / kActSiluMul (rows in gate/up pairs)
     float* workspace;
     uint32_t M, N, K;
+    uint32_t n_width;           // token columns of a tile: a multiple of 16, at most N_TILE (tile_width)
+    uint32_t idesc;             // instruction descriptor of the MMAs, which carries that width
     WorkPlan plan;
     int* status;
 };
@@ -365,7 +367,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                 const uint32_t m_tile = PAIR ? 2u * p_tile + half_id : p_tile;                        // this CTA's 128 rows
                 const uint64_t blk0 = ((uint64_t)m_tile * 2 + half) * kblocks + seg.kb_begin;   // my row block, first K block
                 // a pair splits the tile's token rows: this CTA copies its half
-                const int32_t n0 = (int32_t)((seg.tile - p_tile * plan.n_tiles) * N_TILE + half_id * Cfg::n_local);
+                const int32_t n0 = (int32_t)((seg.tile - p_tile * plan.n_tiles) * p.n_width + half_id * Cfg::n_local);
                 const uint32_t nstages = (seg.nkb + KS - 1) / KS;
                 uint32_t sidx = plan_first_stage(plan, cta, nstages);   // stage of the segment's K range handled next
                 if (warp == kProducerWarp && lane == 0 && issued == 0) PROF_STAMP(14);
@@ -393,7 +395,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                             ptx::tma_load_3d_pair(dst, &act_map, 0, n0, (int32_t)(seg.kb_begin + kb_off), ptx::mapa(bar, 0u), pol);
                         } else if (acts) {
                             // always KS blocks: blocks past the end of K are zero-filled by the copy
-                            ptx::mbar_arrive_expect_tx(bar, KS * Cfg::b_block);
+                            ptx::mbar_arrive_expect_tx(bar, KS * p.n_width * 128u);
                             ptx::tma_load_3d(dst, &act_map, 0, n0, (int32_t)(seg.kb_begin + kb_off), bar, pol);
                         } else {
                             ptx::mbar_arrive_expect_tx(bar, cnt * (Raw::bytes128 / 2));
@@ -427,7 +429,8 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         // stage, each as soon as its slot of the tensor-memory ring is full, and accumulates them in its own
         // accumulator); then all four warps, one per tensor-memory lane quadrant, read the accumulators, add them and
         // store the tile (lane = output channel, column = token).
-        constexpr uint32_t idesc = ptx::idesc_f16_f32(PAIR ? 2 * kTileM : kTileM, N_TILE);
+        const uint32_t idesc = p.idesc;
+        const uint32_t b_step = PAIR ? Cfg::b_block >> 4 : p.n_width * 8u;   // from one K block's activations to the next, in descriptor units
         // In a pair the first CTA issues for both.  The second CTA's issuing warp has nothing to do in the main loop: its
         // activation copies are counted on the first CTA's barrier (a copy may name a barrier of either CTA of the pair) and
         // its unpack warps arrive there too.  (An earlier form had this warp wait for its own copies and pass the news on
@@ -495,10 +498,10 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                                 for (uint32_t kk = 0; kk < 4; kk++) {   // four K=16 steps; B advances 32 bytes inside the swizzle row
                                     if constexpr (PAIR)
                                         ptx::mma_f16_ts_pair_elect(d_tmem, a_tmem + b * kAColsPerKBlock + kk * 8,
-                                                                   b_desc + kbi * (Cfg::b_block >> 4) + kk * 2, idesc, accumulate);
+                                                                   b_desc + kbi * b_step + kk * 2, idesc, accumulate);
                                     else
                                         ptx::mma_f16_ts_elect(d_tmem, a_tmem + b * kAColsPerKBlock + kk * 8,
-                                                              b_desc + kbi * (Cfg::b_block >> 4) + kk * 2, idesc, accumulate);
+                                                              b_desc + kbi * b_step + kk * 2, idesc, accumulate);
                                     accumulate = 1u;
                                 }
                             }
@@ -561,8 +564,8 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
             // issuers that contributed: the fullest stage of the segment holds min(KS, nkb) K blocks, dealt to the issuers in turn
             constexpr int CH = 16;   // columns handled per round
 #pragma unroll 1
-            for (int c0 = 0; c0 < N_TILE; c0 += CH) {
-                const uint32_t n0 = n_tile * N_TILE + c0;
+            for (uint32_t c0 = 0; c0 < p.n_width; c0 += CH) {
+                const uint32_t n0 = n_tile * p.n_width + c0;
                 if (n0 >= p.N) break;
                 uint32_t v[CH];
                 float f[CH];
@@ -587,7 +590,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                         if (n0 + u < p.N) dst[(size_t)u * p.M] = f[u] * row_scale;
                 } else {   // a pair's slot holds the 256 rows of the plan's tile: each CTA its half
                     constexpr uint32_t kSlotRows = PAIR ? 2u * kTileM : (uint32_t)kTileM;
-                    float* dst = p.workspace + ((size_t)seg.out_index * N_TILE + c0) * kSlotRows + half_id * kTileM + row_in_tile;
+                    float* dst = p.workspace + ((size_t)seg.out_index * p.n_width + c0) * kSlotRows + half_id * kTileM + row_in_tile;
 #pragma unroll
                     for (int u = 0; u < CH; u++)
                         if (n0 + u < p.N) dst[u * kSlotRows] = f[u] * row_scale;
@@ -1056,11 +1059,21 @@ static std::atomic<int> g_pair_tiles{0};   // off: measured 0.6 of the single-CT
 void set_pair_tiles(int on) { g_pair_tiles.store(on < 0 ? 0 : (on > 2 ? 2 : on)); }   // 2: also for layers too small to occupy every pair
 int pair_tiles() { return g_pair_tiles.load(); }
 
+// Tokens of a tile: the batch is cut into as few tiles as the kernel's widest allows, all equally wide (rounded up to the 16
+// columns the MMA counts in), instead of full tiles and a remainder that is padded to one: the copies, the MMAs and the
+// epilogue of a tile cost what its columns cost.  333 tokens are two tiles of 176 columns instead of 256: the four layers of a
+// 13B FP5 block 258 -> 216 us (gate/up 108 -> 88 us); below ~200 columns the unpack warps set the pace.
+static size_t gemm_n_tiles(size_t N) { return (N + 255) / 256; }
+static int tile_width(size_t N) {
+    const size_t n_tiles = gemm_n_tiles(N), share = (N + n_tiles - 1) / n_tiles;
+    return (int)((share + 15) / 16 * 16);
+}
+
 // Whether a call runs as CTA pairs on 256-row tiles (the widest tile only, the library's own decomposition, enough row
 // tiles to occupy the pairs), and its plan: for a pair the plan's row tiles are 256 rows and its "CTAs" are pairs.
 static int plan_call(size_t M, size_t N, size_t K, int split_k, bool has_targets, WorkPlan* plan, bool* pair) {
     const int n_tile = gemm_n_tile(N);
-    const size_t n_tiles = (N + n_tile - 1) / n_tile;
+    const size_t n_tiles = gemm_n_tiles(N);
     const int sms = device_sm_count() < (int)kMaxGrid ? device_sm_count() : (int)kMaxGrid;
     *pair = pair_tiles() && n_tile == 256 && split_k == 0 && !has_targets && sms >= 2 &&
             (pair_tiles() == 2 || (M / 256) * n_tiles >= (size_t)(sms / 2));
@@ -1171,14 +1184,14 @@ cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void*
         return cudaErrorMisalignedAddress;
     if (M > 0x7fffffffull || N > 0x7fffffffull || K > 0x7fffffffull) return cudaErrorInvalidValue;
     const int n_tile = gemm_n_tile(N);
-    const size_t n_tiles = (N + n_tile - 1) / n_tile;
-    if ((M / kTileM) * n_tiles > 0x3fffffffull) return cudaErrorInvalidValue;
+    if ((M / kTileM) * gemm_n_tiles(N) > 0x3fffffffull) return cudaErrorInvalidValue;
     Params prm;
     WorkPlan& plan = prm.plan;
     bool pair = false;
     const int eff_split = plan_call(M, N, K, split_k, targets != nullptr, &plan, &pair);
+    const int width = pair ? n_tile : tile_width(N);
     CUtensorMap map;
-    cudaError_t err = make_act_map(&map, act, N, K, pair ? n_tile / 2 : n_tile, gemm_ks(n_tile));   // a pair's CTAs copy half a tile each
+    cudaError_t err = make_act_map(&map, act, N, K, pair ? width / 2 : width, gemm_ks(n_tile));   // a pair's CTAs copy half a tile each
     if (err != cudaSuccess) return err;
 
     prm.weight = static_cast<const uint8_t*>(weight);
@@ -1199,13 +1212,15 @@ cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void*
     prm.M = (uint32_t)M;
     prm.N = (uint32_t)N;
     prm.K = (uint32_t)K;
+    prm.n_width = (uint32_t)width;
+    prm.idesc = ptx::idesc_f16_f32(pair ? 2 * kTileM : kTileM, (uint32_t)width);
     prm.status = status;
     FPX_DISPATCH_FORMAT(e_bits, m_bits, (err = launch_by_n<kE, kM>(n_tile, pair, stream, map, prm)));
     if (err != cudaSuccess) return err;
     if (plan.mode == kStreamK) {
         const uint32_t rem = plan_rem_tiles(plan);
         if (rem == 0) return cudaSuccess;
-        return launch_streamk_fixup(stream, where, workspace, N, n_tile, plan, epilogue, pair ? 2 * kTileM : kTileM);
+        return launch_streamk_fixup(stream, where, workspace, N, width, plan, epilogue, pair ? 2 * kTileM : kTileM);
     }
     if (eff_split > 1) return launch_splitk_reduce(stream, out, workspace, M * N, eff_split, true, M, epilogue);
     return cudaSuccess;

@@ -86,6 +86,16 @@ def test_prefill_like(oracle_mod, bs):
     _check(oracle_mod, f.linear_forward_cuda(x, packed, s, 1), truth)
 
 
+@pytest.mark.parametrize("bs", [33, 47, 48, 49, 65, 80, 81, 113, 129, 144, 145, 241, 257, 272, 289, 333, 481, 513, 530, 769])
+@pytest.mark.parametrize("split_k", [0, 1, 3])
+def test_tile_widths(oracle_mod, bs, split_k):
+    """Batches are cut into equally wide token tiles of any multiple of 16 columns: the last token of a tile, the first of the
+    next, and widths at both ends of every kernel's range, for whole tiles, stream-K slots and the caller's split."""
+    import fp6_llm_b200 as f
+    packed, s, x, truth = _case(oracle_mod, 2, 2, 512, 704, bs, seed=bs)
+    _check(oracle_mod, f.linear_forward_eXmY_cuda(2, 2, x, packed, s, split_k), truth)
+
+
 @pytest.mark.parametrize("e,m", FORMATS)
 def test_known_answer_all_ones_full_size(e, m):
     """Reference tests' all-1.0 words: every output must equal IC exactly, at a full LLaMA-2-70B layer shape."""
