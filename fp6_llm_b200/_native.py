@@ -1,4 +1,5 @@
-"""Builds and loads libfp6_b200.so (the CUDA kernels behind the C interface in include/fp6_llm_b200.h).
+"""Builds and loads libfp6_b200.so (the CUDA kernels behind the C interface in include/fp6_llm_b200.h) and fp6_b200_host.so
+(the layer call on torch tensors, csrc/torch_host.cpp).
 
 The library is compiled in-tree with nvcc for sm_100a only.  There is no fallback of any kind: if the
 library is missing or fails to load, every operator raises.
@@ -6,6 +7,8 @@ library is missing or fails to load, every operator raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -15,6 +18,8 @@ _ROOT = os.path.dirname(_PKG)
 _CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libfp6_b200.so")
+HOST_PATH = os.path.join(LIB_DIR, "fp6_b200_host.so")
+HOST_SOURCE = "torch_host.cpp"
 SOURCES = ("fpx_gemm.cu", "fpx_native.cu", "fpx_prepack.cu", "c_api.cu", "c_api_noalloc.cu")
 HEADERS = ("fpx_codes.cuh", "fpx_epilogue.cuh", "fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
 
@@ -49,27 +54,50 @@ def _nvcc() -> str:
     return cand
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _stale(path: str, sources) -> bool:
+    if not os.path.exists(path):
         return True
-    built = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(_CSRC, f) for f in SOURCES + HEADERS]
+    built = os.path.getmtime(path)
+    deps = [os.path.join(_CSRC, f) for f in sources]
     deps += [os.path.join(_ROOT, "include", f) for f in ("fp6_llm_b200.h", "fp6_llm_b200_cxx.cuh")]
     return any(os.path.getmtime(d) > built for d in deps)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources.  Returns its path."""
-    if not force and not _stale():
-        return LIB_PATH
-    os.makedirs(LIB_DIR, exist_ok=True)
-    cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH]
-    cmd += [os.path.join(_CSRC, s) for s in SOURCES]
+def _run(what: str, cmd) -> str:
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    if verbose:
-        print(res.stderr)
+        raise RuntimeError(f"{what} failed:\n" + res.stdout + res.stderr)
+    return res.stderr
+
+
+def _build_host() -> None:
+    """The Python binding of the layer call: plain C++ against torch's headers, linked to the library beside it."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", HOST_PATH, os.path.join(_CSRC, HOST_SOURCE)]
+    for inc in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
+        cmd += ["-isystem", inc]
+    cmd += ["-L" + os.path.join(root, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            "-L" + LIB_DIR, "-l:" + os.path.basename(LIB_PATH), "-Wl,-rpath,$ORIGIN"]
+    _run("g++", cmd)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compile the library and its Python binding if they are missing or older than their sources.  Returns the library's
+    path."""
+    os.makedirs(LIB_DIR, exist_ok=True)
+    if force or _stale(LIB_PATH, SOURCES + HEADERS):
+        cmd = [_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH]
+        out = _run("nvcc", cmd + [os.path.join(_CSRC, s) for s in SOURCES])
+        if verbose:
+            print(out)
+    if force or _stale(HOST_PATH, (HOST_SOURCE,)):
+        _build_host()
     return LIB_PATH
 
 
@@ -151,6 +179,24 @@ def lib() -> ctypes.CDLL:
     L.fp6b200_device_status.argtypes = [ctypes.POINTER(ci)]
     _lib = L
     return L
+
+
+_host = None
+
+
+def host():
+    """The native host side of the layer call (csrc/torch_host.cpp).  Raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it first (fp6_llm_b200.build()); there is no fallback path")
+        import torch  # noqa: F401  (its libraries must be loaded first)
+        loader = importlib.machinery.ExtensionFileLoader("fp6_b200_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fp6_b200_host", HOST_PATH, loader=loader))
+        loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def check(code: int, what: str) -> None:

@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from .formats import bit_width, check_format, magnitudes
 from .ops import (ACT_NONE, ACT_SILU_MUL, interleave_gate_up, linear_forward_ex, linear_forward_native, native_preferred,
                   native_repack, native_supported, quantize_prepack_cuda, row_scales_cuda)
@@ -21,7 +22,19 @@ def _enable_native(layer) -> None:
     layer.register_buffer("weight_native", native_repack(layer.e_bits, layer.m_bits, layer.weight))
 
 
-def _forward(layer, flat: torch.Tensor, activation: int) -> torch.Tensor:
+def _forward(layer, x: torch.Tensor, activation: int) -> torch.Tensor:
+    held = layer._buffers
+    y = _native.host().layer(layer.e_bits, layer.m_bits, x, held.get("weight"), held.get("weight_native"), held.get("scales"),
+                             layer.split_k, held.get("bias"), activation)
+    if y is not NotImplemented:   # the native host side took the call: contiguous fp16 activations on the weights' device
+        return y
+    if x.dtype != torch.float16 or x.shape[-1] != layer.in_features:
+        raise ValueError(f"expected fp16 activations [..., {layer.in_features}]")
+    flat = x.reshape(-1, layer.in_features).contiguous()
+    return _forward_flat(layer, flat, activation).reshape(*x.shape[:-1], layer.out_features)
+
+
+def _forward_flat(layer, flat: torch.Tensor, activation: int) -> torch.Tensor:
     native = getattr(layer, "weight_native", None)
     if native is not None and layer.split_k == 0 and native_preferred(layer.e_bits, layer.m_bits, layer.weight.shape[0],
                                                                       layer.in_features, flat.shape[0]):
@@ -69,11 +82,7 @@ class FPxLinear(torch.nn.Module):
         return cls(packed, scales, bias, e_bits, m_bits, split_k)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if x.dtype != torch.float16 or x.shape[-1] != self.in_features:
-            raise ValueError(f"expected fp16 activations [..., {self.in_features}]")
-        flat = x.reshape(-1, self.in_features).contiguous()
-        y = _forward(self, flat, ACT_NONE)
-        return y.reshape(*x.shape[:-1], self.out_features)
+        return _forward(self, x, ACT_NONE)
 
     def enable_native(self) -> "FPxLinear":
         """Also keep the weights in the tile layout of the tensor cores' own six-bit inputs (6 more bits per weight,
@@ -122,11 +131,7 @@ class FPxGateUpLinear(torch.nn.Module):
         return cls(packed, scales, bias, e_bits, m_bits, split_k)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        if x.dtype != torch.float16 or x.shape[-1] != self.in_features:
-            raise ValueError(f"expected fp16 activations [..., {self.in_features}]")
-        flat = x.reshape(-1, self.in_features).contiguous()
-        y = _forward(self, flat, ACT_SILU_MUL)
-        return y.reshape(*x.shape[:-1], self.out_features)
+        return _forward(self, x, ACT_SILU_MUL)
 
     def enable_native(self) -> "FPxGateUpLinear":
         """See :meth:`FPxLinear.enable_native`."""

@@ -58,10 +58,9 @@ _retired: list = []
 
 
 def _workspace(device, nbytes: int) -> torch.Tensor:
-    """Grow-only fp32 split-K workspace per (device, stream) (the reference allocates one per call,
-    fp6_llm/csrc/fp6_linear.cu:185-187): calls on one stream run in order and may share it, calls on different
-    streams get their own.  A buffer that is outgrown is kept alive until the process ends, because work already
-    queued (or captured in a CUDA graph) may still use it."""
+    """Grow-only fp32 workspace per (device, stream) of the sharded layer: calls on one stream run in order and may share it,
+    calls on different streams get their own.  A buffer that is outgrown is kept alive until the process ends, because work
+    already queued (or captured in a CUDA graph) may still use it."""
     key = (device, torch.cuda.current_stream(device).cuda_stream)
     ws = _workspaces.get(key)
     if ws is None or ws.numel() * 4 < nbytes:
@@ -84,6 +83,9 @@ ACT_NONE, ACT_SILU_MUL = 0, 1
 
 
 def _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, activation):
+    out = _native.host().linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, activation)
+    if out is not NotImplemented:
+        return out
     _require_cuda()
     check_format(EXPONENT, MANTISSA)
     if _in_feats.dtype != torch.float16 or _scales.dtype != torch.float16 or _weights.dtype != torch.int32:
@@ -114,8 +116,9 @@ def _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, acti
     dev = _in_feats.device
     L = _native.lib()
     with torch.cuda.device(dev):
+        # one workspace per call, as in the reference (fp6_llm/csrc/fp6_linear.cu:185-187)
         nbytes = L.fp6b200_workspace_bytes(OC, B, IC, splitK)
-        ws = _workspace(dev, nbytes) if nbytes else None
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
         out = torch.empty((B, OC // 2 if activation == ACT_SILU_MUL else OC), dtype=torch.float16, device=dev)
         if bias is None and activation == ACT_NONE:
             rc = L.fp6b200_linear(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats),
@@ -196,6 +199,9 @@ def linear_forward_native(EXPONENT: int, MANTISSA: int, _in_feats: torch.Tensor,
     """Out[B, OC] = In[B, IC] @ dequant(W)[OC, IC]^T with the weights in the layout of :func:`native_repack`, for up to
     64 tokens (C: fp6b200_linear_native).  Same result as :func:`linear_forward_ex` up to fp32 summation order: the
     activations enter the tensor cores as four exact e5m2 planes and the six-bit codes as they are."""
+    out = _native.host().native(EXPONENT, MANTISSA, _in_feats, _weights_native, _scales, bias, activation)
+    if out is not NotImplemented:
+        return out
     _require_cuda()
     if _in_feats.dtype != torch.float16 or _scales.dtype != torch.float16 or _weights_native.dtype != torch.uint8:
         raise ValueError("expected fp16 activations, uint8 native weights and fp16 scales")
@@ -219,7 +225,7 @@ def linear_forward_native(EXPONENT: int, MANTISSA: int, _in_feats: torch.Tensor,
         raise ValueError("bias must be a contiguous fp16 tensor with OC elements on the layer's device")
     dev = _in_feats.device
     with torch.cuda.device(dev):
-        ws = _workspace(dev, L.fp6b200_native_workspace_bytes(B, IC))
+        ws = torch.empty(L.fp6b200_native_workspace_bytes(B, IC), dtype=torch.uint8, device=dev)
         out = torch.empty((B, OC // 2 if activation == ACT_SILU_MUL else OC), dtype=torch.float16, device=dev)
         rc = L.fp6b200_linear_native(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights_native), _ptr(_scales),
                                      _ptr(_in_feats), _ptr(out), OC, B, IC, _ptr(ws),

@@ -1,0 +1,123 @@
+"""The native host side of the layer call (csrc/torch_host.cpp) against the Python form of the same operators: it takes plain
+contiguous CUDA tensors and nothing else, and whichever form runs, results, shapes and errors are the same."""
+import threading
+
+import pytest
+import torch
+
+import fp6_llm_b200 as f
+from fp6_llm_b200 import _native
+
+
+@pytest.fixture(scope="module")
+def host(native_lib):
+    return _native.host()
+
+
+def test_declines_what_is_not_a_plain_cuda_call(host):
+    x, w = torch.zeros(2, 64, dtype=torch.float16), torch.zeros(256, 12, dtype=torch.int32)
+    s, tiles = torch.zeros(256, dtype=torch.float16), torch.zeros(2 * 12288, dtype=torch.uint8)
+    assert host.linear(3, 2, x, w, s, 0, None, 0) is NotImplemented          # CPU tensors
+    assert host.native(3, 2, x, tiles, s, None, 0) is NotImplemented
+    assert host.layer(3, 2, x, w, tiles, s, 0, None, 0) is NotImplemented
+    assert host.linear(3, 2, None, w, s, 0, None, 0) is NotImplemented
+    assert host.linear(3.0, 2, x, w, s, 0, None, 0) is NotImplemented
+    assert host.linear(3, 2, x, w, s, 2 ** 70, None, 0) is NotImplemented
+    assert host.linear(3, 2, x) is NotImplemented and host.layer() is NotImplemented
+
+
+def _layer(oc=512, ic=256, e=3, m=2, bias=True, cls=None):
+    gen = torch.Generator(device="cuda").manual_seed(oc + ic)
+    w = torch.randn(oc, ic, generator=gen, device="cuda").half() * 0.02
+    s = f.FPxLinear.row_scales(w, e, m)
+    b = torch.randn(oc, generator=gen, device="cuda").half() if bias else None
+    return (cls or f.FPxLinear)(f.quantize_prepack_cuda(w, s, e, m), s, b, e, m)
+
+
+class _Declining:
+    """Stands in for the binding so that the Python form runs."""
+    linear = native = layer = staticmethod(lambda *a: NotImplemented)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("e,m", [(3, 2), (2, 2), (2, 3), (3, 1), (2, 1)])
+@pytest.mark.parametrize("batch", [1, 8, 32, 33, 70, 150])
+def test_same_as_the_python_form(host, monkeypatch, e, m, batch):
+    for cls in (f.FPxLinear, f.FPxGateUpLinear):
+        for with_bias in (False, True):
+            layer = _layer(e=e, m=m, bias=with_bias, cls=cls)
+            x = torch.randn(batch, 256, device="cuda").half()
+            forms = [x, x.reshape(1, batch, 256), x[0], x.t().contiguous().t(), torch.nn.Parameter(x, requires_grad=False),
+                     torch.cat([x, x], 1)[:, :256], x[::2]]
+            for native in (False, True):
+                if native:
+                    layer.enable_native()
+                got = [layer(t) for t in forms]
+                calls = [lambda: f.linear_forward_ex(e, m, x, layer.weight, layer.scales, 2, layer.bias)]
+                if native and batch <= f.NATIVE_MAX_TOKENS:
+                    calls.append(lambda: f.linear_forward_native(e, m, x, layer.weight_native, layer.scales, layer.bias))
+                got += [c() for c in calls]
+                with monkeypatch.context() as mp:
+                    mp.setattr(_native, "_host", _Declining)
+                    want = [layer(t) for t in forms] + [c() for c in calls]
+                for a, b in zip(got, want):
+                    assert a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype and torch.equal(a, b)
+    assert f.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_same_errors(host):
+    layer = _layer()
+    x = torch.randn(4, 256, device="cuda").half()
+    args = (3, 2, x, layer.weight, layer.scales)
+    for bad in [(x.float(),), (x.cpu(),), (x[:, :128].contiguous(),), (x[:0],), (x[0],), (x.reshape(2, 2, 256),), (x.t(),)]:
+        with pytest.raises(ValueError):
+            f.linear_forward_eXmY_cuda(3, 2, bad[0], layer.weight, layer.scales, 1)
+    with pytest.raises(ValueError):
+        f.linear_forward_eXmY_cuda(*args, -1)
+    with pytest.raises(ValueError):
+        f.linear_forward_eXmY_cuda(4, 3, x, layer.weight, layer.scales, 1)
+    with pytest.raises(ValueError):
+        f.linear_forward_ex(*args, 0, layer.bias[:100])
+    with pytest.raises(ValueError):
+        f.linear_forward_ex(*args, 0, None, 5)
+    with pytest.raises(ValueError):
+        layer(x.float())
+    with pytest.raises(ValueError):
+        layer(x[:, :192])
+    off = torch.empty(4 * 256 + 1, dtype=torch.float16, device="cuda")[1:].reshape(4, 256)   # 2-byte aligned: the library refuses
+    with pytest.raises(RuntimeError, match="fp6b200_linear failed"):
+        f.linear_forward_eXmY_cuda(3, 2, off, layer.weight, layer.scales, 1)
+    with pytest.raises(RuntimeError):   # a batched tensor has no memory of its own
+        torch.func.vmap(layer)(x.reshape(2, 2, 256))
+
+
+@pytest.mark.gpu
+def test_streams_threads_and_graphs(host):
+    """Workspaces belong to a call: several threads on streams of their own, and replayed graphs beside eager calls, do not
+    disturb one another."""
+    layer = _layer(1536, 4096, bias=False).enable_native()
+    xs = [torch.randn(n, 4096, device="cuda").half() for n in (1, 8, 40, 200)]
+    want = [layer(x) for x in xs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()), torch.no_grad():
+            for _ in range(30):
+                got = [layer(x) for x in xs]
+            torch.cuda.current_stream().synchronize()
+            wrong.extend(j for j, (a, b) in enumerate(zip(got, want)) if not torch.equal(a, b))
+
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = [layer(x) for x in xs]
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for _ in range(20):
+        graph.replay()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not wrong and all(torch.equal(a, b) for a, b in zip(captured, want)) and f.device_status() == 0
