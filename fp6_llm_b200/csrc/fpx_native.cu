@@ -60,6 +60,7 @@ constexpr int kNatFirstIssuer = 2;             // warps 2..5: MMA issue (the fir
 constexpr int kNatMaxIssuers = 4;
 constexpr int kNatFirstEpilogue = kNatFirstIssuer + kNatMaxIssuers;   // warps 6..9: one per tensor-memory lane quadrant
 constexpr int kNatFirstConverter = kNatFirstEpilogue + 4;   // warps 10..: split the fp16 activations (fused variant only)
+constexpr uint32_t kNatPrefetch = 12;           // tiles of a CTA asked into L2 before the previous kernel has finished
 constexpr int kNatMaxTokens = 64;               // 4 x 64 = 256 MMA columns
 
 template <int N_TILE>
@@ -100,6 +101,7 @@ struct NatCfg {
 };
 
 struct NatParams {
+    const uint8_t* weights;     // the tiles the weight map describes
     const __half* scales;
     OutTargets out;
     uint32_t weights_static;
@@ -374,6 +376,20 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
     } else {
         // ------------------------------------------------------------ epilogue: one warp per tensor-memory lane quadrant
         const int q = warp & 3;
+        // The first tiles are asked into L2 while the previous kernel of the stream finishes (L2 is where that kernel's stores end
+        // up too, so this reads nothing early): a ring's worth, by the warps that have nothing to do yet.  At one token
+        // 22016 x 4096 15.2 -> 13.8 us, 4096 x 11008 9.6 -> 8.7 us; at 16 tokens 57344 x 8192 60.5 -> 56.8 us.
+        if (!p.weights_static) {
+            SegmentIter ahead;
+            Segment part;
+            plan_start(plan, cta, &ahead);
+            uint32_t seen = 0;
+            while (seen < kNatPrefetch && plan_next(plan, cta, &ahead, &part))
+                for (uint32_t i = 0; i < part.nkb && seen < kNatPrefetch; i++, seen++)
+                    if ((seen & 3u) == (uint32_t)q && ptx::elect_one())
+                        ptx::bulk_prefetch_l2(p.weights + ((size_t)part.tile * p.ktiles + part.kb_begin + i) * kNatTileBytes, kNatTileBytes);
+            __syncwarp();
+        }
         asm volatile("griddepcontrol.wait;" ::: "memory");   // before the scales are read and anything is stored
         uint32_t nseg = 0, j0 = 0;
         bool ok = true;
@@ -673,6 +689,7 @@ cudaError_t launch_native_gemm(int e_bits, int m_bits, cudaStream_t stream, cons
     // 2. the GEMM
     const int sms = device_sm_count() < 256 ? device_sm_count() : 256;
     NatParams prm;
+    prm.weights = static_cast<const uint8_t*>(weight_native);
     prm.scales = scales;
     prm.out = where;
     prm.weights_static = (uint32_t)weights_static();

@@ -170,6 +170,11 @@ __device__ __forceinline__ void bulk_g2s(uint32_t smem_dst, const void* gmem_src
         ::"r"(smem_dst), "l"(gmem_src), "r"(bytes), "r"(bar), "l"(policy)
         : "memory");
 }
+// Asks L2 for `bytes` (a multiple of 16) from a 16-byte aligned address.  Nothing is read on behalf of the program: a write
+// to the same memory that completes later is seen by every later load.
+__device__ __forceinline__ void bulk_prefetch_l2(const void* gmem_src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(gmem_src), "r"(bytes) : "memory");
+}
 // 3-D tiled tensor copy global -> shared through a tensor map; x is the innermost coordinate.
 __device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int32_t x, int32_t y, int32_t z,
                                             uint32_t bar, uint64_t policy) {

@@ -86,6 +86,30 @@ def test_prefill_like(oracle_mod, bs):
     _check(oracle_mod, f.linear_forward_cuda(x, packed, s, 1), truth)
 
 
+@pytest.mark.parametrize("native", [False, True])
+@pytest.mark.parametrize("bs", [1, 8, 20])
+def test_weights_written_just_before(bs, native):
+    """Weights that the previous kernel of the stream writes: the layer asks L2 for them before that kernel has finished, and
+    must still see what it wrote."""
+    import fp6_llm_b200 as f
+    gen = torch.Generator(device="cuda").manual_seed(bs)
+    oc, ic = 2048, 4096
+    s = torch.full((oc,), 0.01, dtype=torch.float16, device="cuda")
+    x = torch.randn(bs, ic, generator=gen, device="cuda").half()
+    sources = []
+    for _ in range(3):
+        w = f.quantize_prepack_cuda(torch.randn(oc, ic, generator=gen, device="cuda").half() * 0.1, s)
+        sources.append(f.native_repack(3, 2, w) if native else w)
+    run = (lambda w: f.linear_forward_native(3, 2, x, w, s)) if native else (lambda w: f.linear_forward_cuda(x, w, s, 0))
+    want = [run(w) for w in sources]
+    held = torch.empty_like(sources[0])
+    got = []
+    for i in range(12):
+        held.copy_(sources[i % 3])
+        got.append(run(held))
+    assert all(torch.equal(y, want[i % 3]) for i, y in enumerate(got)) and f.device_status() == 0
+
+
 @pytest.mark.parametrize("bs", [33, 47, 48, 49, 65, 80, 81, 113, 129, 144, 145, 241, 257, 272, 289, 333, 481, 513, 530, 769])
 @pytest.mark.parametrize("split_k", [0, 1, 3])
 def test_tile_widths(oracle_mod, bs, split_k):
