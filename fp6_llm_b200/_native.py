@@ -33,7 +33,7 @@ C_SYMBOLS = (
     "fp6b200_dequant", "fp6b200_dequant_host", "fp6b200_dequant_packed", "fp6b200_splitk_reduce",
     "fp6b200_device_status", "fp6b200_linear_static_scratch", "fp6b200_static_scratch_bytes",
     "fp6b200_linear_gather", "fp6b200_set_option", "fp6b200_get_option", "fp6b200_quantize_prepack", "fp6b200_row_scales",
-    "fp6b200_linear_host_io_batch", "fp6b200_kernel_launches", "fp6b200_linear_ex",
+    "fp6b200_linear_host_io_batch", "fp6b200_kernel_launches", "fp6b200_linear_ex", "fp6b200_linear_scratch",
     "fp6b200_native_supported", "fp6b200_native_preferred", "fp6b200_native_weight_bytes", "fp6b200_native_workspace_bytes",
     "fp6b200_native_repack", "fp6b200_linear_native", "fp6b200_native_kernel_launches", "fp6b200_linear_native_gather",
 )
@@ -123,6 +123,8 @@ def lib() -> ctypes.CDLL:
     L.fp6b200_linear.argtypes = [ci, ci, vp, vp, vp, vp, vp, sz, sz, sz, vp, ci]
     L.fp6b200_linear_ex.restype = ci
     L.fp6b200_linear_ex.argtypes = [ci, ci, vp, vp, vp, vp, vp, sz, sz, sz, vp, ci, vp, ci]
+    L.fp6b200_linear_scratch.restype = ci
+    L.fp6b200_linear_scratch.argtypes = [ci, ci, vp, vp, vp, vp, vp, sz, sz, sz, vp, vp, vp, ci]
     L.fp6b200_native_supported.restype = ci
     L.fp6b200_native_supported.argtypes = [ci, ci, sz, sz, sz]
     L.fp6b200_native_preferred.restype = ci

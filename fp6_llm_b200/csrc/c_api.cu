@@ -151,6 +151,21 @@ int fp6b200_linear_ex(int e_bits, int m_bits, void* stream, const void* weight_p
                             static_cast<__half*>(out), M, N, K, workspace, split_k, status, nullptr, &epi);
 }
 
+int fp6b200_linear_scratch(int e_bits, int m_bits, void* stream, const void* weight_packed, const void* scales, const void* act,
+                           void* out, size_t M, size_t N, size_t K, void* (*get_scratch)(void*, size_t), void* context, const void* bias,
+                           int activation) {
+    int* status = status_ptr();
+    if (!status) return cudaErrorInitializationError;
+    if (!get_scratch) return cudaErrorInvalidValue;
+    fpx::Epilogue epi;
+    epi.bias = static_cast<const __half*>(bias);
+    epi.activation = activation;
+    const fpx::Scratch scratch = {get_scratch, context};
+    return fpx::launch_gemm(e_bits, m_bits, static_cast<cudaStream_t>(stream), weight_packed,
+                            static_cast<const __half*>(scales), static_cast<const __half*>(act),
+                            static_cast<__half*>(out), M, N, K, nullptr, 0, status, nullptr, &epi, &scratch);
+}
+
 int fp6b200_native_supported(int e_bits, int m_bits, size_t M, size_t N, size_t K) {
     return fpx::native_format(e_bits, m_bits) && M > 0 && M % 256 == 0 && K > 0 && K % 64 == 0 && N > 0 &&
            N <= (size_t)fpx::native_max_tokens();

@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "fpx_internal.h"
+#include "ptx_sm100.cuh"
 
 namespace fpx {
 
@@ -87,6 +88,43 @@ __device__ __forceinline__ void store_columns(const OutTargets& out, int activat
             const uint32_t n = n1 + 4u * j;
             if (n < N) *reinterpret_cast<uint2*>(dst + (size_t)n * out.ld) = v[j];
         }
+    }
+}
+
+// Four finished rows m0 .. m0 + 3 (m0 a multiple of 4) of token n: bias, activation, fp16, memory.
+__device__ __forceinline__ void store_four_rows(const OutTargets& out, int activation, const __half* bias, float4 acc, uint32_t m0,
+                                                uint32_t n) {
+    if (bias) {
+        acc.x += __half2float(bias[m0]); acc.y += __half2float(bias[m0 + 1]);
+        acc.z += __half2float(bias[m0 + 2]); acc.w += __half2float(bias[m0 + 3]);
+    }
+    if (activation == kActSiluMul) {   // two gate/up pairs -> two output channels
+        *reinterpret_cast<uint32_t*>(out.ptr[0] + (size_t)n * out.ld + out.row0 + (m0 >> 1)) =
+            pack_half2(silu_mul(acc.x, acc.y), silu_mul(acc.z, acc.w));
+        return;
+    }
+    const uint2 packed = make_uint2(pack_half2(acc.x, acc.y), pack_half2(acc.z, acc.w));
+    const size_t at = (size_t)n * out.ld + out.row0 + m0;
+    for (uint32_t t = 0; t < out.count; t++) *reinterpret_cast<uint2*>(out.ptr[t] + at) = packed;
+}
+
+// End of a tile whose K range a cluster shared: every CTA holds its part as [token][128 rows] fp32 at `part` of its shared
+// memory (the pipeline ring, idle by then); the warps of all CTAs take a token each in turn and add the parts in rank order.
+// Called by whole warps between the two cluster barriers.
+__device__ __forceinline__ void reduce_cluster(const OutTargets& out, int activation, const __half* bias, uint32_t part, uint32_t ctas,
+                                               uint32_t rank, uint32_t warps, uint32_t row0, uint32_t n0, uint32_t tokens, int warp,
+                                               int lane) {
+    for (uint32_t t = (uint32_t)warp * ctas + rank; t < tokens; t += warps * ctas) {
+        const uint32_t addr = part + (t * 128u + 4u * (uint32_t)lane) * 4u;
+        float4 v[kMaxCluster];
+#pragma unroll
+        for (uint32_t s = 0; s < (uint32_t)kMaxCluster; s++)
+            if (s < ctas) v[s] = ptx::ld_cluster_f4(ptx::mapa(addr, s));
+        float4 acc = v[0];
+#pragma unroll
+        for (uint32_t s = 1; s < (uint32_t)kMaxCluster; s++)
+            if (s < ctas) { acc.x += v[s].x; acc.y += v[s].y; acc.z += v[s].z; acc.w += v[s].w; }
+        store_four_rows(out, activation, bias, acc, row0 + 4u * (uint32_t)lane, n0 + t);
     }
 }
 

@@ -612,6 +612,10 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
 #pragma unroll
                     for (int u = 0; u < CH; u++)
                         if (n0 + u < p.N) dst[(size_t)u * p.M] = f[u] * row_scale;
+                } else if (seg.out_kind == kOutClusterPart) {   // into the ring, which is idle: this is the CTA's last segment
+#pragma unroll
+                    for (int u = 0; u < CH; u++)
+                        if (n0 + u < p.N) ptx::sts_f32(ring + ((c0 + u) * kTileM + row_in_tile) * 4u, f[u] * row_scale);
                 } else {   // a pair's slot holds the 256 rows of the plan's tile: each CTA its half
                     constexpr uint32_t kSlotRows = PAIR ? 2u * kTileM : (uint32_t)kTileM;
                     float* dst = p.workspace + ((size_t)seg.out_index * p.n_width + c0) * kSlotRows + half_id * kTileM + row_in_tile;
@@ -745,6 +749,23 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         PROF_FLUSH();
     }
 
+    const bool clustered = !PAIR && plan.mode == kCluster;   // the same for the whole grid
+    if (clustered) {   // remainder tile r = cluster r: every thread of the cluster comes by here, whatever it gave up on
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // not every role has
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        const uint32_t r = cta / plan.cluster;
+        if (r < plan.rem_tiles) {
+            const uint32_t tile = plan.full_waves * plan.grid + r, m_tile = tile / plan.n_tiles, n0 = (tile - m_tile * plan.n_tiles) * p.n_width;
+            const uint32_t tokens = p.N - n0 < p.n_width ? p.N - n0 : p.n_width;
+            reduce_cluster(p.out, (int)p.activation, p.bias, ring, plan.cluster, cta - r * plan.cluster, kWarps, m_tile * kTileM, n0, tokens,
+                           warp, lane);
+        }
+        __syncwarp();
+        ptx::cluster_arrive();
+    }
+
     // ------------------------------------------------------------ teardown
     ptx::tc_fence_before_sync();
     __syncthreads();
@@ -760,6 +781,8 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         else ptx::tmem_dealloc(tmem_base, kTmemCols);
     }
     if (threadIdx.x == 0 && *abort_word != 0) atomicCAS(p.status, 0, *abort_word);
+    __syncwarp();
+    if (clustered) ptx::cluster_wait();   // a peer may still be reading this CTA's part
     if (threadIdx.x == 0) PROF_STAMP(9);
 }
 
@@ -805,7 +828,6 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(__half* __restrict__
 // round trips cost more than this launch, and wide tiles are then summed by one SM instead of all.)
 constexpr int kFixupThreads = 512;   // 16 (column, group) pairs of 32 threads
 constexpr uint64_t kEvenGridMinPercent = 85;
-constexpr uint64_t kFixupCostUnits = 20;   // the fix-up launch and its dependency cost about as much as 20 K blocks on one CTA
 constexpr uint64_t kMinUnitsPerCta = 8;   // a CTA is not started for fewer 64-K blocks than this (two 256-K stages)
 __global__ void __launch_bounds__(kFixupThreads) streamk_fixup_kernel(const __grid_constant__ OutTargets out, const float* __restrict__ slots,
                                                                          uint32_t N, int n_tile_size, const __grid_constant__ WorkPlan plan,
@@ -868,22 +890,7 @@ __global__ void __launch_bounds__(kFixupThreads) streamk_fixup_kernel(const __gr
             const float4 v = group_sum[g * cols + col][threadIdx.x & 31u];
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        const uint32_t m0 = m_tile * tile_rows + row_off;
-        if (bias) {
-            acc.x += __half2float(bias[m0]); acc.y += __half2float(bias[m0 + 1]);
-            acc.z += __half2float(bias[m0 + 2]); acc.w += __half2float(bias[m0 + 3]);
-        }
-        if (activation == kActSiluMul) {   // two gate/up pairs -> two output channels
-            const __half2 r2 = __floats2half2_rn(silu_mul(acc.x, acc.y), silu_mul(acc.z, acc.w));
-            *reinterpret_cast<__half2*>(out.ptr[0] + (size_t)n * out.ld + out.row0 + (m0 >> 1)) = r2;
-        } else {
-            __half2 lo = __floats2half2_rn(acc.x, acc.y), hi = __floats2half2_rn(acc.z, acc.w);
-            uint2 packed;
-            packed.x = *reinterpret_cast<uint32_t*>(&lo);
-            packed.y = *reinterpret_cast<uint32_t*>(&hi);
-            const size_t at = (size_t)n * out.ld + out.row0 + m0;
-            for (uint32_t t = 0; t < out.count; t++) *reinterpret_cast<uint2*>(out.ptr[t] + at) = packed;
-        }
+        store_four_rows(out, activation, bias, acc, m_tile * tile_rows + row_off, n);
     }
     if (threadIdx.x == 0 && blockIdx.y == 0) PROF_STAMP(12);
 }
@@ -961,35 +968,74 @@ cudaError_t make_act_map(CUtensorMap* map, const __half* act, size_t N, size_t K
 
 }  // namespace
 
-// The work decomposition of one call (see WorkPlan): split_k == 0 is the library's own (data-parallel waves of tiles,
-// then the K blocks of the remaining tiles dealt out evenly), split_k >= 1 the caller's.  Returns the effective split.
-int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, WorkPlan* out) {
+// The work decomposition of one call (see WorkPlan).  split_k == 0: the library's own, the one of
+//   whole tiles  one CTA each, when there are no more tiles than SMs (nothing is split);
+//   clusters     waves of whole tiles, the remaining ones shared by clusters of 2 .. 8 CTAs each;
+//   stream-K     waves of whole tiles, the K blocks of the remaining ones dealt out evenly, a fix-up kernel behind (only with
+//                a workspace for the slots)
+// that the costs say is done first: a phase takes as long as its busiest CTA, or as long as memory needs for its weights.
+// split_k >= 1: the caller's.  Returns the effective split.
+int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, const PlanCosts& costs, bool slots, bool clusters_ok, WorkPlan* out) {
     WorkPlan& plan = *out;
     plan.m_tiles = (uint32_t)(M / kTileM);
     plan.n_tiles = (uint32_t)n_tiles;
     plan.kblocks = (uint32_t)(K / kKBlock);
+    plan.cluster = 1;
     const uint64_t tiles = (uint64_t)plan.m_tiles * plan.n_tiles;
     int eff_split = 1;
     if (split_k == 0) {
-        plan.mode = kStreamK;
         plan.split_k = 1;
         const uint64_t units = tiles * plan.kblocks;
-        // Fewer tiles than SMs: one CTA per whole tile (no tile is split, so no fix-up kernel follows) when that costs no
-        // more than dealing the K blocks out evenly plus the fix-up, which is worth about kFixupCostUnits K blocks.
-        if (tiles <= (uint64_t)sms && plan.kblocks <= units / (uint64_t)sms + kFixupCostUnits) {
+        const double kb = (double)plan.kblocks;
+        const auto phase = [&](double blocks_per_cta, double blocks) {
+            const double sm = blocks_per_cta * costs.unit, mem = blocks * costs.unit_gpu;
+            return sm > mem ? sm : mem;
+        };
+        double best = 1e300;
+        if (tiles <= (uint64_t)sms) {
+            plan.mode = kStreamK;
             plan.grid = (uint32_t)tiles;
-            plan_finalize(&plan);
-            return eff_split;
+            best = phase(kb, (double)units);
         }
-        uint64_t cap = units / kMinUnitsPerCta;     // CTAs that still get kMinUnitsPerCta blocks each, at least one per tile
-        if (cap < tiles) cap = tiles;
-        if (cap > (uint64_t)sms) cap = (uint64_t)sms;
-        plan.grid = (uint32_t)cap;
-        // Fewer tiles than SMs: a grid that is a multiple of the tile count gives every tile the same number of
-        // CTAs and no CTA a second tile (one epilogue per CTA); taken when it still fills most of the SMs.
-        if (tiles < cap) {
-            const uint64_t even = tiles * (cap / tiles);
-            if (even * 100 >= cap * kEvenGridMinPercent) plan.grid = (uint32_t)even;
+        if (slots) {
+            uint64_t cap = units / kMinUnitsPerCta;     // CTAs that still get kMinUnitsPerCta blocks each, at least one per tile
+            if (cap < tiles) cap = tiles;
+            if (cap > (uint64_t)sms) cap = (uint64_t)sms;
+            bool aligned = false;
+            // Fewer tiles than SMs: a grid that is a multiple of the tile count gives every tile the same number of
+            // CTAs and no CTA a second tile (one epilogue per CTA); taken when it still fills most of the SMs.
+            if (tiles < cap) {
+                const uint64_t even = tiles * (cap / tiles);
+                if (even * 100 >= cap * kEvenGridMinPercent) cap = even, aligned = true;
+            }
+            const double cost = phase((double)units / (double)cap, (double)units) + (tiles % cap ? costs.fixup : 0.0) +
+                                (aligned || tiles % cap == 0 ? 0.0 : costs.segment);
+            if (cost < best) {
+                best = cost;
+                plan.mode = kStreamK;
+                plan.grid = (uint32_t)cap;
+            }
+        }
+        for (int c = 2; clusters_ok && c <= kMaxCluster && (uint64_t)c * 4 <= plan.kblocks; c++) {
+            const uint64_t room = (uint64_t)max_clusters(c), fit = (uint64_t)(sms / c), clusters = room < fit ? room : fit;
+            if (clusters == 0) continue;
+            const uint64_t waves = tiles / (clusters * c), rem = tiles - waves * clusters * c;
+            if (rem > clusters || rem == 0) continue;
+            // with waves before it, a size that does not divide the SM groups evenly waits for its SMs to come free together:
+            // 57344 x 8192 at 64 tokens, native path 61.5 us with three, 57.9 with two
+            if (waves && (c & (c - 1))) continue;
+            const double cost = phase(kb * (double)waves, (double)(waves * clusters * c) * kb) +
+                                phase((double)((plan.kblocks + c - 1) / c), (double)rem * kb) + costs.reduce + (waves ? costs.segment : 0.0);
+            if (cost < best) {
+                best = cost;
+                plan.mode = kCluster;
+                plan.cluster = (uint32_t)c;
+                plan.grid = (uint32_t)((waves ? clusters : rem) * c);
+            }
+        }
+        if (best == 1e300) {   // no workspace, more tiles than SMs and no cluster fits the remainder: waves of whole tiles
+            plan.mode = kClassic;
+            plan.grid = (uint32_t)sms;
         }
     } else {              // the caller's split: splits beyond the number of K blocks would be empty
         plan.mode = kClassic;
@@ -1029,9 +1075,9 @@ cudaError_t launch_one(cudaStream_t stream, const CUtensorMap& map, const Params
     attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch() ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (PAIR) {
+    if (PAIR || prm.plan.mode == kCluster) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = 2;
+        attr[1].val.clusterDim.x = PAIR ? 2 : prm.plan.cluster;
         attr[1].val.clusterDim.y = 1;
         attr[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
@@ -1079,6 +1125,36 @@ int device_sm_count() {
     return n;
 }
 
+// The kernels here take a whole SM's shared memory each, so any of them gives the answer.
+int max_clusters(int ctas) {
+    static std::atomic<int> known[64][kMaxCluster + 1];   // 0: not asked yet, else 1 + the answer
+    int dev = 0;
+    if (ctas < 1 || ctas > kMaxCluster || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    int n = known[dev][ctas].load(std::memory_order_relaxed);
+    if (n) return n - 1;
+    auto kernel = fpx_gemm_kernel<3, 2, 64>;
+    constexpr uint32_t smem = Config<6, 64>::smem_bytes;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int found = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&found, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        found = 0;
+    }
+    known[dev][ctas].store(found + 1, std::memory_order_relaxed);
+    return found;
+}
+
 static std::atomic<int> g_pair_tiles{0};   // off: measured 0.6 of the single-CTA speed (see Config)
 void set_pair_tiles(int on) { g_pair_tiles.store(on < 0 ? 0 : (on > 2 ? 2 : on)); }   // 2: also for layers too small to occupy every pair
 int pair_tiles() { return g_pair_tiles.load(); }
@@ -1095,14 +1171,38 @@ static int tile_width(size_t N) {
 
 // Whether a call runs as CTA pairs on 256-row tiles (the widest tile only, the library's own decomposition, enough row
 // tiles to occupy the pairs), and its plan: for a pair the plan's row tiles are 256 rows and its "CTAs" are pairs.
+// Microseconds, measured on the layers of 7B and 70B models (4096 x 4096 .. 57344 x 8192, 1 .. 256 tokens) with each
+// decomposition forced in turn; 64-wide K blocks of 128 rows, six bits per weight.  Against the fix-up kernel a cluster's shared
+// memory saves 0.5 us at one token and 4 at 256 (8192 x 8192: 15.2 -> 14.5 us at 16 tokens, 22.9 -> 20.7 at 128, 34.0 -> 30.7 at
+// 256; 8192 x 28672 at 256 tokens 92.2 -> 88.3), and whole tiles beat both while two thirds of the SMs have one (12288 x 4096: 14.6
+// -> 12.2 us at 16 tokens, 22.5 -> 18.3 at 128; with 80 tiles of 148 they lose, 18.6 against 20.4 us).
+static PlanCosts plan_costs(size_t N) {
+    const int n_tile = gemm_n_tile(N), width = tile_width(N);
+    PlanCosts c;
+    c.unit = n_tile <= 64 ? 0.145 : (width > 160 ? 0.00125 * width : 0.2);
+    c.unit_gpu = 6144 / 6.3e6;
+    c.fixup = 4.3;
+    c.reduce = 1.5 + 0.01 * width;
+    c.segment = 1.5;
+    return c;
+}
 static int plan_call(size_t M, size_t N, size_t K, int split_k, bool has_targets, WorkPlan* plan, bool* pair) {
     const int n_tile = gemm_n_tile(N);
     const size_t n_tiles = gemm_n_tiles(N);
     const int sms = device_sm_count() < (int)kMaxGrid ? device_sm_count() : (int)kMaxGrid;
     *pair = pair_tiles() && n_tile == 256 && split_k == 0 && !has_targets && sms >= 2 &&
             (pair_tiles() == 2 || (M / 256) * n_tiles >= (size_t)(sms / 2));
-    if (*pair) return make_plan(M / 2, n_tiles, K, split_k, sms / 2, plan);   // M / 2 rows in 128-row tiles = M in 256-row tiles
-    return make_plan(M, n_tiles, K, split_k, sms, plan);
+    const PlanCosts costs = plan_costs(N);
+    if (*pair) return make_plan(M / 2, n_tiles, K, split_k, sms / 2, costs, true, false, plan);   // M / 2 rows in 128-row tiles = M in 256-row tiles
+    if (split_k == 0) return make_plan(M, n_tiles, K, 0, sms, costs, true, true, plan);
+    // The caller's split is taken as the offer of its workspace, split_k * M * N partial sums (none for 1): the library's own
+    // decomposition runs wherever it needs no more.  With the reference's heuristic (12 splits) 5120 x 13824 e2m2 at 16 tokens
+    // takes 21.3 us split as asked and 15.1 us this way; 4096 x 4096 at 8 tokens, not split, 10.9 against 8.2 us.
+    const size_t slots = 2 * (size_t)sms * kTileM * tile_width(N);
+    const bool room = split_k > 1 && (size_t)split_k * M * N >= slots;
+    make_plan(M, n_tiles, K, 0, sms, costs, room, true, plan);
+    if (plan->mode != kClassic) return 1;
+    return make_plan(M, n_tiles, K, split_k, sms, costs, false, false, plan);
 }
 
 int gemm_kernel_launches(size_t M, size_t N, size_t K, int split_k) {
@@ -1151,7 +1251,7 @@ int programmatic_launch() { return g_programmatic_launch.load(); }
 cudaError_t launch_streamk_fixup(cudaStream_t stream, const OutTargets& where, const float* workspace, size_t N,
                                  int n_tile, const WorkPlan& plan, const Epilogue* epilogue, int tile_rows) {
     const uint32_t rem = plan_rem_tiles(plan);
-    if (rem == 0) return cudaSuccess;
+    if (rem == 0 || plan.mode != kStreamK) return cudaSuccess;
     // groups: as many as half the parts of a tile (about grid / rem CTAs share one), while the grid stays within ~2 CTAs per SM
     const uint32_t parts = (plan.grid + rem - 1) / rem + 1;
     uint32_t groups = 1;
@@ -1177,7 +1277,7 @@ cudaError_t launch_streamk_fixup(cudaStream_t stream, const OutTargets& where, c
 
 cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void* weight, const __half* scales,
                         const __half* act, __half* out, size_t M, size_t N, size_t K, float* workspace, int split_k,
-                        int* status, const OutTargets* targets, const Epilogue* epilogue) {
+                        int* status, const OutTargets* targets, const Epilogue* epilogue, const Scratch* scratch) {
     if (!format_supported(e_bits, m_bits)) return cudaErrorInvalidValue;
     const __half* bias = epilogue ? epilogue->bias : nullptr;
     const int activation = epilogue ? epilogue->activation : kActNone;
@@ -1202,7 +1302,7 @@ cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void*
     }
     if (M == 0 || M % 256 != 0 || K == 0 || K % 64 != 0 || N == 0 || split_k < 0 || split_k > 65535)
         return cudaErrorInvalidValue;
-    if (!weight || !scales || !act || !out || (split_k != 1 && !workspace)) return cudaErrorInvalidValue;
+    if (!weight || !scales || !act || !out || (split_k != 1 && !workspace && !scratch)) return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(weight) & 15) || (reinterpret_cast<uintptr_t>(act) & 15) ||
         (reinterpret_cast<uintptr_t>(out) & 7) || (reinterpret_cast<uintptr_t>(workspace) & 15))
         return cudaErrorMisalignedAddress;
@@ -1213,7 +1313,13 @@ cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void*
     WorkPlan& plan = prm.plan;
     bool pair = false;
     const int eff_split = plan_call(M, N, K, split_k, targets != nullptr, &plan, &pair);
+
     const int width = pair ? n_tile : tile_width(N);
+    if (!workspace && scratch && plan.mode == kStreamK && plan_rem_tiles(plan)) {
+        workspace = static_cast<float*>(scratch->get(scratch->context, gemm_auto_workspace_bytes(N)));
+        if (!workspace) return cudaErrorMemoryAllocation;
+        if (reinterpret_cast<uintptr_t>(workspace) & 15) return cudaErrorMisalignedAddress;
+    }
     CUtensorMap map;
     cudaError_t err = make_act_map(&map, act, N, K, pair ? width / 2 : width, gemm_ks(n_tile));   // a pair's CTAs copy half a tile each
     if (err != cudaSuccess) return err;

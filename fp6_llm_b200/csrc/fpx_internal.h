@@ -50,17 +50,33 @@ struct Epilogue {
     int activation;
 };
 
+// A workspace that is asked for only when a call turns out to need one; get returns nullptr when there is none.
+struct Scratch {
+    void* (*get)(void* context, size_t bytes);
+    void* context;
+};
 // GEMM (+ split-K reduction when split_k > 1).  All pointers are device pointers.  targets == nullptr: the result
 // goes to out[N][M] (out[N][M / 2] with kActSiluMul); otherwise out is ignored (split_k must then be 0 or 1, and no
 // activation).  epilogue == nullptr: plain layer.
 cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void* weight, const __half* scales,
                         const __half* act, __half* out, size_t M, size_t N, size_t K, float* workspace, int split_k,
-                        int* status, const OutTargets* targets = nullptr, const Epilogue* epilogue = nullptr);
+                        int* status, const OutTargets* targets = nullptr, const Epilogue* epilogue = nullptr,
+                        const Scratch* scratch = nullptr);
 // Work decomposition of one call over `sms` CTAs (see WorkPlan): M rows in 128-row tiles, K in 64-wide blocks;
-// split_k == 0 is the library's own (waves of whole tiles, then the K blocks of the remaining tiles dealt out evenly),
+// split_k == 0 is the library's own: whichever of its decompositions the costs (microseconds) say is done first,
 // split_k >= 1 the caller's.  Returns the effective split.
 struct WorkPlan;
-int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, WorkPlan* out);
+struct PlanCosts {
+    double unit;        // a K block of a tile on one CTA, when nothing but the SM limits it
+    double unit_gpu;    // the same block's share of the time memory needs for it, over the whole GPU
+    double fixup;       // the fix-up kernel behind the GEMM
+    double reduce;      // the end of a tile that a cluster shares
+    double segment;     // a CTA turning from one segment to the next
+};
+constexpr int kMaxCluster = 8;
+int max_clusters(int ctas);   // clusters of that many CTAs the current device holds at once, one CTA per SM; 0 if none
+// slots: there is a workspace for stream-K parts; clusters_ok: the kernel can end a tile inside a cluster
+int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, const PlanCosts& costs, bool slots, bool clusters_ok, WorkPlan* out);
 // tile_rows: height of the plan's row tiles (128, or 256 when CTA pairs computed them)
 cudaError_t launch_streamk_fixup(cudaStream_t stream, const OutTargets& where, const float* workspace, size_t N,
                                  int n_tile, const WorkPlan& plan, const Epilogue* epilogue, int tile_rows = 128);

@@ -295,9 +295,12 @@ FPX_HD void split_range(uint32_t k_blocks, uint32_t splits, uint32_t z, uint32_t
 //             [c*U/grid, (c+1)*U/grid) of the remainder.  A CTA's first and last remainder segment may
 //             cover only part of a tile's K range; those go to partial slots 2c and 2c+1 and a fix-up
 //             kernel sums the slots of every split tile in CTA order.
-enum WorkMode : uint32_t { kClassic = 0, kStreamK = 1 };
+//   kCluster  whole waves as above, then remainder tile r is computed by the CTAs of cluster r, each a share of its K range
+//             (split_range); the parts meet in the cluster's shared memory, so there are no slots and no second kernel.
+//             `cluster` CTAs each, rem_tiles * cluster <= grid, cluster <= kblocks.
+enum WorkMode : uint32_t { kClassic = 0, kStreamK = 1, kCluster = 2 };
 constexpr uint32_t kPlanTableGrid = 256;   // largest grid for which a plan carries its table of remainder starts
-enum OutKind : uint32_t { kOutDirect = 0, kOutSplitPartial = 1, kOutSlotPartial = 2 };
+enum OutKind : uint32_t { kOutDirect = 0, kOutSplitPartial = 1, kOutSlotPartial = 2, kOutClusterPart = 3 };
 
 struct WorkPlan {
     uint32_t mode;
@@ -314,6 +317,7 @@ struct WorkPlan {
     // CTA c starts in the remainder (c == grid: the end), so that a CTA finds its work with two loads.
     uint32_t has_table;
     uint32_t rem_start[kPlanTableGrid + 1];
+    uint32_t cluster;     // kCluster only
 };
 
 struct Segment {
@@ -321,7 +325,7 @@ struct Segment {
     uint32_t kb_begin;
     uint32_t nkb;         // > 0
     uint32_t out_kind;
-    uint32_t out_index;   // split index (kOutSplitPartial) or slot (kOutSlotPartial)
+    uint32_t out_index;   // split index (kOutSplitPartial), slot (kOutSlotPartial) or rank in the cluster (kOutClusterPart)
 };
 
 FPX_HD uint32_t plan_tiles(const WorkPlan& p) { return p.m_tiles * p.n_tiles; }
@@ -333,9 +337,17 @@ FPX_HD void plan_finalize(WorkPlan* p) {
     p->rem_units32 = (units + 1) * p->grid <= 0xffffffffull ? (uint32_t)units : 0u;
     p->has_table = 0;
     if (p->mode == kStreamK && p->grid <= kPlanTableGrid && p->kblocks < 65536u) {
+        // floor(c * units / grid) as (tile, K block), carried along without a division per CTA: a call makes its plan anew
+        const uint32_t tile_step = (uint32_t)(units / p->grid / p->kblocks), kb_step = (uint32_t)(units / p->grid % p->kblocks);
+        const uint32_t part = (uint32_t)(units % p->grid);
+        uint32_t tile = 0, kb = 0, carry = 0;
         for (uint32_t c = 0; c <= p->grid; c++) {
-            const uint64_t u = plan_rem_begin(*p, c);
-            p->rem_start[c] = ((uint32_t)(u / p->kblocks) << 16) | (uint32_t)(u % p->kblocks);
+            p->rem_start[c] = (tile << 16) | kb;
+            carry += part;
+            kb += kb_step + (carry >= p->grid ? 1u : 0u);
+            carry -= carry >= p->grid ? p->grid : 0u;
+            tile += tile_step + (kb >= p->kblocks ? 1u : 0u);
+            kb -= kb >= p->kblocks ? p->kblocks : 0u;
         }
         p->has_table = 1;
     }
@@ -398,6 +410,16 @@ FPX_HD bool plan_next(const WorkPlan& p, uint32_t cta, SegmentIter* it, Segment*
         seg->out_kind = kOutDirect;
         seg->out_index = 0;
         it->step++;
+        return true;
+    }
+    if (p.mode == kCluster) {
+        const uint32_t r = cta / p.cluster;
+        if (it->step > waves || r >= p.rem_tiles) return false;
+        it->step++;
+        seg->tile = waves * p.grid + r;
+        seg->out_kind = kOutClusterPart;
+        seg->out_index = cta - r * p.cluster;
+        split_range(p.kblocks, p.cluster, seg->out_index, &seg->kb_begin, &seg->nkb);
         return true;
     }
     if (it->cur_tile == it->end_tile && it->cur_kb >= it->end_kb) return false;

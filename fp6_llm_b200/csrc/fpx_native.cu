@@ -468,6 +468,10 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
 #pragma unroll
                     for (int u = 0; u < CH; u++) f[u] = f[u] * row_scale + row_bias;
                     store_columns(p.out, (int)p.activation, f, n0, p.N, row, lane);
+                } else if (seg.out_kind == kOutClusterPart) {   // into the ring, which is idle: this is the CTA's last segment
+#pragma unroll
+                    for (int u = 0; u < CH; u++)
+                        if (n0 + u < p.N) ptx::sts_f32(ring + ((t0 + u) * kNatTileM + row_in_tile) * 4u, f[u] * row_scale);
                 } else {   // part of a tile: fp32, scaled, into this CTA's slot [tokens][128]
                     float* dst = p.workspace + ((size_t)seg.out_index * T + t0) * kNatTileM + row_in_tile;
 #pragma unroll
@@ -483,8 +487,22 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         }
     }
 
-    // ------------------------------------------------------------ teardown
     if (threadIdx.x == 0) NAT_STAMP(5);   // roles done
+    const bool clustered = plan.mode == kCluster;   // the same for the whole grid
+    if (clustered) {   // remainder tile r = cluster r: every thread of the cluster comes by here, whatever it gave up on
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // not every role has
+        __syncwarp();
+        ptx::cluster_arrive();
+        ptx::cluster_wait();
+        const uint32_t r = cta / plan.cluster;
+        if (r < plan.rem_tiles)
+            reduce_cluster(p.out, (int)p.activation, p.bias, ring, plan.cluster, cta - r * plan.cluster, Cfg::warps,
+                           (plan.full_waves * plan.grid + r) * kNatTileM, 0, p.N, warp, lane);
+        __syncwarp();
+        ptx::cluster_arrive();
+    }
+
+    // ------------------------------------------------------------ teardown
     ptx::tc_fence_before_sync();
     __syncthreads();
     if (warp == kNatFirstIssuer) {
@@ -497,6 +515,8 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         ptx::tmem_dealloc(tmem_base, Cfg::tmem_cols);
     }
     if (threadIdx.x == 0 && *abort_word != 0) atomicCAS(p.status, 0, *abort_word);
+    __syncwarp();
+    if (clustered) ptx::cluster_wait();   // a peer may still be reading this CTA's part
     if (threadIdx.x == 0) NAT_STAMP(6);   // exit
 }
 
@@ -576,11 +596,18 @@ cudaError_t launch_native_one(cudaStream_t stream, const CUtensorMap& w_map, con
     cfg.blockDim = dim3(NatCfg<N_TILE>::threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = programmatic_launch() ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (prm.plan.mode == kCluster) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = prm.plan.cluster;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
     return cudaLaunchKernelEx(&cfg, kernel, w_map, x_map, prm);
 }
 
@@ -603,6 +630,20 @@ static size_t native_planes_bytes(size_t N, size_t K) {
 size_t native_workspace_bytes(size_t N, size_t K) {
     const size_t ctas = device_sm_count() < 256 ? device_sm_count() : 256;
     return native_planes_bytes(N, K) + 2 * ctas * kNatTileM * (native_n_tile(N) / kPieces) * sizeof(float);
+}
+
+// Units of the plan = K tiles of 128.  Costs in microseconds, found as those of fpx_gemm.cu; the unit is what a stage's bytes
+// take to pass through shared memory twice.  Against the fix-up kernel at 16 tokens: 4096 x 4096 8.5 -> 7.0 us, 4096 x 11008
+// 12.0 -> 10.6, 8192 x 28672 31.7 -> 30.0; at one token 0.2 us either way.
+static void native_plan(size_t M, size_t N, size_t ktiles, int sms, WorkPlan* plan) {
+    const int n_tile = native_n_tile(N);
+    PlanCosts c;
+    c.unit = n_tile <= 16 ? 0.15 : (n_tile <= 32 ? 0.17 : (n_tile <= 64 ? 0.2 : (n_tile <= 128 ? 0.27 : 0.33)));
+    c.unit_gpu = kNatTileBytes / 6.3e6;
+    c.fixup = 3.5;
+    c.reduce = 1.5 + 0.01 * (double)N;
+    c.segment = 0.5;
+    make_plan(M, 1, ktiles * kKBlock, 0, sms, c, true, true, plan);
 }
 
 cudaError_t launch_native_gemm(int e_bits, int m_bits, cudaStream_t stream, const void* weight_native, const __half* scales,
@@ -703,7 +744,7 @@ cudaError_t launch_native_gemm(int e_bits, int m_bits, cudaStream_t stream, cons
     prm.ktiles = (uint32_t)ktiles;
     prm.a_format = e_bits == 3 ? ptx::kFmtE3M2 : ptx::kFmtE2M3;
     prm.status = status;
-    make_plan(M, 1, ktiles * kKBlock, 0, sms, &prm.plan);   // units of the plan = K tiles
+    native_plan(M, N, ktiles, sms, &prm.plan);   // units of the plan = K tiles
     cudaError_t err;
     switch (n_tile) {
         case 16:  err = launch_native_one<16>(stream, w_map, x_map, prm); break;
@@ -721,8 +762,8 @@ int native_kernel_launches(size_t M, size_t N, size_t K) {
     if (M == 0 || M % 256 != 0 || K == 0 || K % 64 != 0 || N == 0 || N > (size_t)kNatMaxTokens) return 0;
     const int sms = device_sm_count() < 256 ? device_sm_count() : 256;
     WorkPlan plan;
-    make_plan(M, 1, native_ktiles(K) * kKBlock, 0, sms, &plan);
-    return (native_n_tile(N) <= 16 ? 1 : 2) + (plan_rem_tiles(plan) ? 1 : 0);
+    native_plan(M, N, native_ktiles(K), sms, &plan);
+    return (native_n_tile(N) <= 16 ? 1 : 2) + (plan.mode == kStreamK && plan_rem_tiles(plan) ? 1 : 0);
 }
 
 }  // namespace fpx

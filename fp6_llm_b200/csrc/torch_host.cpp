@@ -18,7 +18,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <optional>
+#include <exception>
 
 #include "../../include/fp6_llm_b200.h"
 
@@ -56,6 +56,23 @@ struct Call {
     const at::Tensor *x = nullptr, *weight = nullptr, *native = nullptr, *scales = nullptr, *bias = nullptr;
 };
 
+// The workspace of one call, allocated when it is asked for.  Called from C: an exception (out of memory) waits in `failed`.
+struct Workspace {
+    at::TensorOptions options;
+    at::Tensor memory;
+    std::exception_ptr failed;
+    static void* get(void* self, size_t bytes) noexcept {
+        Workspace* w = static_cast<Workspace*>(self);
+        try {
+            w->memory = at::empty({(int64_t)bytes}, w->options);
+            return w->memory.data_ptr();
+        } catch (...) {
+            w->failed = std::current_exception();
+            return nullptr;
+        }
+    }
+};
+
 PyObject* fail(const char* what, int rc) {
     const char* msg = fp6b200_error_string(rc);
     PyErr_Format(PyExc_RuntimeError, "%s failed: CUDA error %d (%s)", what, rc, msg ? msg : "?");
@@ -85,21 +102,20 @@ PyObject* run(const Call& c, bool last_dim_only) {
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     c10::DimVector sizes(x.sizes());
     sizes[dim - 1] = c.activation == kSiluMul ? oc / 2 : oc;
-    const auto on_device = at::TensorOptions().device(x.device());
-    at::Tensor out = at::empty(sizes, on_device.dtype(at::kHalf));
+    at::Tensor out = at::empty(sizes, at::TensorOptions().device(x.device()).dtype(at::kHalf));
     // The workspace goes back to the allocator when this returns; the stream orders whoever gets it next behind these kernels.
-    const size_t bytes = c.native ? fp6b200_native_workspace_bytes(batch, ic) : fp6b200_workspace_bytes(oc, batch, ic, c.split_k);
-    at::Tensor ws;
-    if (bytes) ws = at::empty({(int64_t)bytes}, on_device.dtype(at::kByte));
+    Workspace ws{at::TensorOptions().device(x.device()).dtype(at::kByte), {}, nullptr};
     void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
     const void* bias = c.bias ? c.bias->data_ptr() : nullptr;
-    void *xp = x.data_ptr(), *op = out.data_ptr(), *sp = c.scales->data_ptr(), *wsp = bytes ? ws.data_ptr() : nullptr;
+    void *xp = x.data_ptr(), *op = out.data_ptr(), *sp = c.scales->data_ptr();
     void* wp = c.native ? c.native->data_ptr() : c.weight->data_ptr();
-    int rc;
+    void* planes = c.native ? Workspace::get(&ws, fp6b200_native_workspace_bytes(batch, ic)) : nullptr;
+    int rc = 0;
     Py_BEGIN_ALLOW_THREADS   // a full launch queue blocks
-    if (c.native) rc = fp6b200_linear_native(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, wsp, bias, c.activation);
-    else rc = fp6b200_linear_ex(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, static_cast<float*>(wsp), c.split_k, bias, c.activation);
+    if (!c.native) rc = fp6b200_linear_scratch(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, &Workspace::get, &ws, bias, c.activation);
+    else if (planes) rc = fp6b200_linear_native(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, planes, bias, c.activation);
     Py_END_ALLOW_THREADS
+    if (ws.failed) std::rethrow_exception(ws.failed);
     if (rc != 0) return fail(c.native ? "fp6b200_linear_native" : "fp6b200_linear", rc);
     return THPVariable_Wrap(std::move(out));
 }

@@ -117,16 +117,11 @@ def _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, acti
     L = _native.lib()
     with torch.cuda.device(dev):
         # one workspace per call, as in the reference (fp6_llm/csrc/fp6_linear.cu:185-187)
-        nbytes = L.fp6b200_workspace_bytes(OC, B, IC, splitK)
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+        # and with it the library's own split of K, whatever the caller names
+        ws = torch.empty(L.fp6b200_workspace_bytes(OC, B, IC, 0), dtype=torch.uint8, device=dev)
         out = torch.empty((B, OC // 2 if activation == ACT_SILU_MUL else OC), dtype=torch.float16, device=dev)
-        if bias is None and activation == ACT_NONE:
-            rc = L.fp6b200_linear(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats),
-                                  _ptr(out), OC, B, IC, _ptr(ws) if ws is not None else None, splitK)
-        else:
-            rc = L.fp6b200_linear_ex(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats),
-                                     _ptr(out), OC, B, IC, _ptr(ws) if ws is not None else None, splitK,
-                                     _ptr(bias) if bias is not None else None, activation)
+        rc = L.fp6b200_linear_ex(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats),
+                                 _ptr(out), OC, B, IC, _ptr(ws), 0, _ptr(bias) if bias is not None else None, activation)
     _native.check(rc, "fp6b200_linear")
     return out
 
@@ -137,7 +132,7 @@ def linear_forward_eXmY_cuda(EXPONENT: int, MANTISSA: int, _in_feats: torch.Tens
     fp6_llm/csrc/fp6_linear.cu:269-313).
 
     _in_feats  fp16 [B, IC] cuda;  _weights  int32 [OC, IC/32*(1+E+M)] cuda, prepacked;
-    _scales    fp16 [OC] cuda;     splitK >= 1 as in the reference, 0 = let the library choose.
+    _scales    fp16 [OC] cuda;     splitK >= 0: accepted as in the reference; how K is split is the library's choice.
     Runs on the current torch stream (the reference uses the legacy default stream)."""
     return _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, None, ACT_NONE)
 

@@ -57,6 +57,16 @@ int fp6b200_linear_ex(int e_bits, int m_bits, void* stream, const void* weight_p
                       void* out, size_t M, size_t N, size_t K, float* workspace, int split_k, const void* bias, int activation);
 
 /*
+ * fp6b200_linear_ex with split_k == 0 for callers whose workspace costs something to get: get_scratch(context, bytes) is called
+ * at most once, before anything is launched, and only if the decomposition of this call needs a workspace (most small layers'
+ * does not).  It returns device memory, 16-byte aligned, that stays valid until the call's kernels have run, or NULL (the call then
+ * returns cudaErrorMemoryAllocation).  It must not throw.  (No counterpart in the reference.)
+ */
+int fp6b200_linear_scratch(int e_bits, int m_bits, void* stream, const void* weight_packed, const void* scales, const void* act,
+                           void* out, size_t M, size_t N, size_t K, void* (*get_scratch)(void* context, size_t bytes), void* context,
+                           const void* bias, int activation);
+
+/*
  * The layer on the tensor cores' own six-bit inputs, for batches of up to 64 tokens (no
  * counterpart in the reference, whose kernel - like fp6b200_linear - rebuilds an fp16 pattern of every weight with integer
  * instructions before the MMA: fp6_llm/csrc/include/utils_parallel_dequant.cuh:24-63).  sm_100's tensor cores multiply

@@ -161,6 +161,36 @@ int harness_check_plan(uint32_t mode, uint32_t m_tiles, uint32_t n_tiles, uint32
     return 0;
 }
 
+// The same for remainder tiles shared by clusters of `ctas` CTAs: whole tiles stored directly, every other tile covered by the
+// ranks of one cluster in order, each as its CTA's last segment, and nothing left for a fix-up kernel.
+int harness_check_cluster_plan(uint32_t m_tiles, uint32_t n_tiles, uint32_t kblocks, uint32_t grid, uint32_t ctas) {
+    WorkPlan p{kCluster, m_tiles, n_tiles, kblocks, 1, grid, 0, 0, 0};
+    p.cluster = ctas;
+    plan_finalize(&p);
+    const uint32_t tiles = plan_tiles(p), rem = plan_rem_tiles(p);
+    std::vector<uint32_t> cover((size_t)tiles * kblocks, 0);
+    for (uint32_t c = 0; c < grid; c++) {
+        SegmentIter it;
+        plan_start(p, c, &it);
+        Segment s;
+        bool shared = false;
+        while (plan_next(p, c, &it, &s)) {
+            if (shared) return 1;                       // the shared tile must come last
+            if (s.nkb == 0 || s.tile >= tiles || s.kb_begin + s.nkb > kblocks) return 2;
+            for (uint32_t k = 0; k < s.nkb; k++) cover[(size_t)s.tile * kblocks + s.kb_begin + k]++;
+            if (s.out_kind == kOutDirect) {
+                if (s.nkb != kblocks) return 3;
+            } else {
+                shared = true;
+                if (s.out_kind != kOutClusterPart || s.out_index != c % ctas) return 4;
+                if (s.tile != p.full_waves * grid + c / ctas) return 5;   // where the reduction looks for it
+            }
+        }
+        if (shared != (c / ctas < rem)) return 6;
+    }
+    for (uint32_t v : cover) if (v != 1) return 7;
+    return 0;
+}
 
 // Codes of n quotients, as the fused quantise + pack kernel computes them.
 void harness_quantize(int e_bits, int m_bits, const float* q, int n, unsigned char* codes) {

@@ -1,0 +1,85 @@
+"""How a layer's tiles and K blocks are dealt to the SMs: whole tiles, clusters that share a tile and add their parts in shared
+memory, stream-K parts behind a fix-up kernel, and the caller's own split through the C interface.  Every route against a
+64-bit product of the dequantised weights: fp16 output rounding is 2^-11 / sqrt(3) = 2.8e-4 in the 2-norm, the fp32 sums add
+less than 1e-5."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+REL = 4e-4
+
+
+def _layer(oc, ic, bs, e, m):
+    import fp6_llm_b200 as f
+    gen = torch.Generator(device="cuda").manual_seed(oc + ic + bs)
+    w = torch.randn(oc, ic, generator=gen, device="cuda").half() * 0.02
+    s = f.FPxLinear.row_scales(w, e, m)
+    packed = f.quantize_prepack_cuda(w, s, e, m)
+    codes = f.dequant_packed_cuda(e, m, packed, torch.ones_like(s)).double() * s.double()[:, None]
+    x = torch.randn(bs, ic, generator=gen, device="cuda").half()
+    bias = torch.randn(oc, generator=gen, device="cuda").half()
+    return packed, s, x, bias, x.double() @ codes.T
+
+
+def _rel(y, truth):
+    return ((y.double() - truth).norm() / truth.norm()).item()
+
+
+# one tile; K too short to share; odd K shares; few tiles and a long K; a tile per SM and two over; more, with a short K
+SHAPES = [(256, 64), (256, 512), (512, 1088), (1280, 5120), (4096, 704), (5120, 2112), (12288, 512), (19200, 2048), (19200, 128),
+          (37888 + 512, 576)]
+
+
+@pytest.mark.parametrize("oc,ic", SHAPES)
+@pytest.mark.parametrize("bs", [1, 5, 16, 40, 100, 130, 300])
+def test_every_decomposition(oc, ic, bs):
+    import fp6_llm_b200 as f
+    packed, s, x, bias, plain = _layer(oc, ic, bs, 3, 2)
+    full = plain + bias.double()
+    gated = torch.nn.functional.silu(full[:, 0::2]) * full[:, 1::2]
+    assert _rel(f.linear_forward_cuda(x, packed, s, 0), plain) < REL
+    assert _rel(f.linear_forward_ex(3, 2, x, packed, s, 0, bias), full) < REL
+    assert _rel(f.linear_forward_ex(3, 2, x, packed, s, 0, bias, f.ACT_SILU_MUL), gated) < REL
+    if bs <= f.NATIVE_MAX_TOKENS:
+        tiles = f.native_repack(3, 2, packed)
+        assert _rel(f.linear_forward_native(3, 2, x, tiles, s), plain) < REL
+        assert _rel(f.linear_forward_native(3, 2, x, tiles, s, bias, f.ACT_SILU_MUL), gated) < REL
+    assert f.device_status() == 0
+
+
+@pytest.mark.parametrize("oc,ic,bs", [(512, 1088, 5), (4096, 704, 16), (1280, 5120, 70), (19200, 2048, 3), (768, 2048, 300)])
+@pytest.mark.parametrize("split_k", [1, 2, 3, 12, 40])
+def test_callers_split_stays_in_its_workspace(native_lib, oc, ic, bs, split_k):
+    """split_k * M * N floats are what the caller owns, whatever decomposition runs; none for split_k = 1."""
+    import fp6_llm_b200 as f
+    packed, s, x, _, plain = _layer(oc, ic, bs, 2, 2)
+    elems = split_k * oc * bs if split_k > 1 else 0
+    held = torch.full((elems + 4096,), -7.0, device="cuda")
+    out = torch.empty(bs, oc, dtype=torch.float16, device="cuda")
+    assert native_lib.fp6b200_linear(2, 2, torch.cuda.current_stream().cuda_stream, packed.data_ptr(), s.data_ptr(), x.data_ptr(),
+                                     out.data_ptr(), oc, bs, ic, held.data_ptr() if elems else None, split_k) == 0
+    assert _rel(out, plain) < REL and bool((held[elems:] == -7.0).all()) and f.device_status() == 0
+    assert native_lib.fp6b200_kernel_launches(oc, bs, ic, split_k) in (1, 2)
+
+
+def test_scratch_is_asked_for_only_when_needed(native_lib):
+    import ctypes
+    import fp6_llm_b200 as f
+    asked = []
+    get_t = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)
+    for (oc, ic, bs), needs in {(1024, 1024, 4): False, (10240, 8192, 4): True}.items():
+        packed, s, x, _, plain = _layer(oc, ic, bs, 3, 2)
+        ws = torch.empty(native_lib.fp6b200_workspace_bytes(oc, bs, ic, 0), dtype=torch.uint8, device="cuda")
+        out = torch.empty(bs, oc, dtype=torch.float16, device="cuda")
+
+        def call(answer):
+            del asked[:]
+            get = get_t(lambda ctx, n: asked.append(n) or answer)
+            return native_lib.fp6b200_linear_scratch(3, 2, torch.cuda.current_stream().cuda_stream, packed.data_ptr(), s.data_ptr(),
+                                                     x.data_ptr(), out.data_ptr(), oc, bs, ic, ctypes.cast(get, ctypes.c_void_p), None,
+                                                     None, 0)
+        assert call(ws.data_ptr()) == 0 and len(asked) == int(needs) and all(n <= ws.numel() for n in asked)
+        assert _rel(out, plain) < REL
+        if needs:
+            assert call(None) == 2   # cudaErrorMemoryAllocation, nothing launched
+    assert f.device_status() == 0

@@ -76,6 +76,22 @@ def test_work_plans_cover_every_unit_once(harness):
     assert n > 1000
 
 
+def test_cluster_plans_cover_every_unit_once(harness):
+    n = 0
+    for tiles, nt in ((1, 1), (2, 1), (3, 1), (32, 1), (86, 1), (172, 1), (448, 1), (64, 2), (5, 9)):
+        for kb in (8, 9, 31, 64, 172):
+            for ctas in range(2, 9):
+                for clusters in (1, 2, 18, 24, 36, 49, 74):
+                    waves = tiles * nt // (clusters * ctas)
+                    rem = tiles * nt - waves * clusters * ctas
+                    if rem == 0 or rem > clusters or ctas > kb:
+                        continue
+                    grid = (clusters if waves else rem) * ctas
+                    assert harness.harness_check_cluster_plan(tiles, nt, kb, grid, ctas) == 0, (tiles, nt, kb, grid, ctas)
+                    n += 1
+    assert n > 200
+
+
 @pytest.mark.parametrize("e,m", ALL_FORMATS)
 def test_quantiser_matches_the_tensor_quantiser(harness, e, m):
     """The scalar round-to-nearest routine of the fused quantise + pack kernel against formats.quantize_rtn, on random
