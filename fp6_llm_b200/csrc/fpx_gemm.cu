@@ -62,13 +62,12 @@ constexpr int gemm_ks(int n_tile) { return n_tile <= 64 ? 4 : (n_tile <= 128 ? 2
 
 constexpr int kTileM = 128;
 constexpr int kAColsPerKBlock = 32;      // 64 fp16 along K per tensor-memory lane
-constexpr int kMaxIssuers = 4;           // warps 0..3: MMA issuers (whole warps, one elected lane) and, one per lane quadrant, the epilogue
+constexpr int kMaxIssuers = 4;           // warps 0..3: MMA issuers (whole warps, one elected lane) and, for narrow tiles, one per lane quadrant, the epilogue
 constexpr int kProducerWarp = 4;         // warps 4,5: the weights' copy producers (whole warps, one elected lane)
 constexpr int kProducerWarps = 2;
 constexpr int kFirstDequantWarp = kProducerWarp + kProducerWarps;
 constexpr int kDequantGroups = 4;        // a group = 4 consecutive warps, one per tensor-memory lane quadrant
 constexpr int kDequantWarps = 4 * kDequantGroups;
-constexpr int kEpilogueWarps = 4;        // = warps 0..3
 constexpr int kActProducerWarp = kFirstDequantWarp + kDequantWarps;   // the last warp: activation copies (one thread)
 constexpr int kWarps = kActProducerWarp + 1;
 constexpr int kThreads = kWarps * 32;
@@ -153,6 +152,8 @@ struct Config {
                   "a slot is always consumed by the same issuing warp");
     static_assert(issuers <= kMaxIssuers, "issuing warps are the first warps of the CTA");
     static constexpr int readers = 4 * pos_per_stage;   // unpack warps that read a stage's weights
+    static constexpr bool unpack_ends = N_TILE >= 64;   // who ends a segment: the unpack warps, or the four issuing warps
+    static constexpr int epilogue_warps = unpack_ends ? kDequantWarps : kMaxIssuers;
     static constexpr uint32_t poll_producer = N_TILE <= 64 ? kPollProducerNarrow : kPollWide;
     static constexpr uint32_t poll_issuer = N_TILE <= 64 ? kPollIssuerNarrow : kPollWide;
     // the unpack warps of a wide tile are ahead of the tensor pipe most of the time: every poll they save is power for it
@@ -303,10 +304,10 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
             ptx::mbar_init(b_empty + 8 * i, Cfg::stage_issuers);
         }
         for (int i = lane; i < SA; i += 32) { ptx::mbar_init(a_full + 8 * i, 4); ptx::mbar_init(a_empty + 8 * i, 1); }
-        if (lane == 0) { ptx::mbar_init(acc_full, NI); ptx::mbar_init(acc_empty, kEpilogueWarps); }
+        if (lane == 0) { ptx::mbar_init(acc_full, NI); ptx::mbar_init(acc_empty, Cfg::epilogue_warps); }
         if constexpr (PAIR) {
             for (int i = lane; i < SA; i += 32) ptx::mbar_init(a_peer + 8 * i, 4);
-            if (lane == 0) ptx::mbar_init(acc_peer, kEpilogueWarps);
+            if (lane == 0) ptx::mbar_init(acc_peer, Cfg::epilogue_warps);
         }
         if (lane == 0) *abort_word = 0;
         ptx::fence_barrier_init();
@@ -334,6 +335,92 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
     if constexpr (PAIR) ptx::cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
     if (threadIdx.x == 0) PROF_STAMP(1);
     const uint32_t tmem_base = *tmem_holder;   // valid for every warp but the producers, which never use it
+
+    // The end of a segment, for the four or sixteen warps of Config::epilogue_warps: read the accumulators (rounds of 16 columns,
+    // `first`, `first + step`, ... for this warp), add them, scale, store.  `has_data`: the issuers that hold a sum.
+    auto end_segment = [&](uint32_t tile, uint32_t out_kind, uint32_t out_index, uint32_t has_data, uint32_t parity, uint32_t first,
+                           uint32_t step) -> bool {
+        const int q = warp & 3;                                   // tensor-memory lane quadrant this warp may touch
+        if constexpr (Cfg::unpack_ends) asm volatile("griddepcontrol.wait;" ::: "memory");   // before the scales are read and anything is stored
+        const uint32_t p_tile = plan.n_tiles == 1 ? tile : tile / plan.n_tiles, n_tile = tile - p_tile * plan.n_tiles;
+        const uint32_t m_tile = PAIR ? 2u * p_tile + half_id : p_tile;   // this CTA's 128 rows of the plan's row tile
+        const uint32_t row_in_tile = 32u * q + lane;
+        const uint32_t row = m_tile * kTileM + row_in_tile;
+        // the accumulator holds sum(x * pattern); pattern = code value / 2^bias, so scale by 2^bias * scale[row] here, in fp32
+        const float row_scale = __half2float(p.scales[row]) * (float)(1u << (16 - (1 << (E_BITS - 1))));
+        const float row_bias = p.bias ? __half2float(p.bias[row]) : 0.0f;   // added where a tile is finished: here, or in the fix-up / reduction
+        if (!ptx::mbar_wait_warp(acc_full, parity, abort_word, kErrAccFull)) return false;
+        if (warp == (Cfg::unpack_ends ? kFirstDequantWarp : 0) && lane == 0) PROF_STAMP(7);
+        ptx::tc_fence_after_sync();
+        const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + Cfg::acc_col0;
+        constexpr int CH = 16;   // columns handled per round
+#pragma unroll 1
+        for (uint32_t c0 = first * CH; c0 < p.n_width; c0 += step * CH) {
+            const uint32_t n0 = n_tile * p.n_width + c0;
+            if (n0 >= p.N) break;
+            uint32_t v[CH];
+            float f[CH];
+#pragma unroll
+            for (int u = 0; u < CH; u++) f[u] = 0.0f;
+#pragma unroll
+            for (uint32_t i = 0; i < (uint32_t)NI; i++)
+                if ((has_data >> i) & 1u) {
+                    ptx::tmem_ld_cols<CH>(acc + i * Cfg::acc_stride + c0, v);
+                    ptx::tc_wait_ld();
+#pragma unroll
+                    for (int u = 0; u < CH; u++) f[u] += __uint_as_float(v[u]);
+                }
+            if (out_kind == kOutDirect) {
+#pragma unroll
+                for (int u = 0; u < CH; u++) f[u] = f[u] * row_scale + row_bias;
+                store_columns(p.out, (int)p.activation, f, n0, p.N, row, lane);
+            } else if (out_kind == kOutSplitPartial) {
+                float* dst = p.workspace + ((size_t)out_index * p.N + n0) * p.M + row;
+#pragma unroll
+                for (int u = 0; u < CH; u++)
+                    if (n0 + u < p.N) dst[(size_t)u * p.M] = f[u] * row_scale;
+            } else if (out_kind == kOutClusterPart) {   // into the ring, which is idle: this is the CTA's last segment
+#pragma unroll
+                for (int u = 0; u < CH; u++)
+                    if (n0 + u < p.N) ptx::sts_f32(ring + ((c0 + u) * kTileM + row_in_tile) * 4u, f[u] * row_scale);
+            } else {   // a pair's slot holds the 256 rows of the plan's tile: each CTA its half
+                constexpr uint32_t kSlotRows = PAIR ? 2u * kTileM : (uint32_t)kTileM;
+                float* dst = p.workspace + ((size_t)out_index * p.n_width + c0) * kSlotRows + half_id * kTileM + row_in_tile;
+#pragma unroll
+                for (int u = 0; u < CH; u++)
+                    if (n0 + u < p.N) dst[u * kSlotRows] = f[u] * row_scale;
+            }
+        }
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (PAIR && half_id != 0u) ptx::mbar_arrive_remote_elected(ptx::mapa(acc_peer, 0u));   // tell the issuing CTA
+        else ptx::mbar_arrive_elected(acc_empty);
+        if (warp == (Cfg::unpack_ends ? kFirstDequantWarp : 0) && lane == 0) PROF_STAMP(8);
+        return true;
+    };
+    // Which issuers hold a sum for a segment that starts at the CTA's running stage j0: issuer i visited the stages t = t_first
+    // (mod issuer_step); with two or more visits one of them was a full stage, with one visit its first position must
+    // hold a K block.
+    auto issuers_with_sum = [&](uint32_t j0, uint32_t nkb, uint32_t nstages) -> uint32_t {
+        uint32_t has_data = 0;
+        {
+            constexpr uint32_t PPS = (uint32_t)Cfg::pos_per_stage, IST = (uint32_t)Cfg::issuer_step;
+            const uint32_t first_stage = plan_first_stage(plan, cta, nstages);
+#pragma unroll
+            for (uint32_t i = 0; i < (uint32_t)NI; i++) {
+                const uint32_t t_first = ((i / PPS) % IST + IST - (j0 % IST)) % IST;
+                bool has = t_first < nstages;
+                if (has && t_first + IST >= nstages) {
+                    uint32_t only = first_stage + t_first;
+                    if (only >= nstages) only -= nstages;
+                    const uint32_t cnt = nkb - only * KS;   // >= KS for every stage but the last of the K range
+                    has = (i % PPS) * (uint32_t)Cfg::kpw < cnt;
+                }
+                has_data |= (has ? 1u : 0u) << i;
+            }
+        }
+        return has_data;
+    };
 
     if (is_producer) {
         // ------------------------------------------------------------ producers (a warp each, one elected lane issues): warps 4 and 5 copy the
@@ -465,7 +552,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
             }
             __syncwarp();
         }
-        asm volatile("griddepcontrol.wait;" ::: "memory");   // before the scales are read and anything is stored
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // nothing to issue before the activations are there
         uint32_t j0 = 0, nseg = 0;
         bool ok = true;
         SegmentIter iter;
@@ -553,82 +640,9 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
-            // Which issuers hold a sum for this segment: issuer i visited the stages t = t_first (mod issuer_step); with two
-            // or more visits one of them was a full stage, with one visit its first position must hold a K block.
-            uint32_t has_data = 0;
-            {
-                constexpr uint32_t PPS = (uint32_t)Cfg::pos_per_stage, IST = (uint32_t)Cfg::issuer_step;
-                const uint32_t first_stage = plan_first_stage(plan, cta, nstages);
-#pragma unroll
-                for (uint32_t i = 0; i < (uint32_t)NI; i++) {
-                    const uint32_t t_first = ((i / PPS) % IST + IST - (j0 % IST)) % IST;
-                    bool has = t_first < nstages;
-                    if (has && t_first + IST >= nstages) {
-                        uint32_t only = first_stage + t_first;
-                        if (only >= nstages) only -= nstages;
-                        const uint32_t cnt = seg.nkb - only * KS;   // >= KS for every stage but the last of the K range
-                        has = (i % PPS) * (uint32_t)Cfg::kpw < cnt;
-                    }
-                    has_data |= (has ? 1u : 0u) << i;
-                }
-            }
+            if constexpr (!Cfg::unpack_ends)
+                if (!end_segment(seg.tile, seg.out_kind, seg.out_index, issuers_with_sum(j0, seg.nkb, nstages), nseg & 1u, 0u, 1u)) break;
             j0 += nstages;
-
-            const uint32_t p_tile = plan.n_tiles == 1 ? seg.tile : seg.tile / plan.n_tiles, n_tile = seg.tile - p_tile * plan.n_tiles;
-            const uint32_t m_tile = PAIR ? 2u * p_tile + half_id : p_tile;   // this CTA's 128 rows of the plan's row tile
-            const uint32_t row_in_tile = 32u * q + lane;
-            const uint32_t row = m_tile * kTileM + row_in_tile;
-            // the accumulator holds sum(x * pattern); pattern = code value / 2^bias, so scale by 2^bias * scale[row] here, in fp32
-            const float row_scale = __half2float(p.scales[row]) * (float)(1u << (16 - (1 << (E_BITS - 1))));
-            const float row_bias = p.bias ? __half2float(p.bias[row]) : 0.0f;   // added where a tile is finished: here, or in the fix-up / reduction
-            if (!PROF_WAIT(5, ptx::mbar_wait_warp(acc_full, nseg & 1u, abort_word, kErrAccFull))) { ok = false; break; }
-            if (threadIdx.x == 0) PROF_STAMP(7);
-            ptx::tc_fence_after_sync();
-            const uint32_t acc = tmem_base + ((uint32_t)(32 * q) << 16) + Cfg::acc_col0;
-            // issuers that contributed: the fullest stage of the segment holds min(KS, nkb) K blocks, dealt to the issuers in turn
-            constexpr int CH = 16;   // columns handled per round
-#pragma unroll 1
-            for (uint32_t c0 = 0; c0 < p.n_width; c0 += CH) {
-                const uint32_t n0 = n_tile * p.n_width + c0;
-                if (n0 >= p.N) break;
-                uint32_t v[CH];
-                float f[CH];
-#pragma unroll
-                for (int u = 0; u < CH; u++) f[u] = 0.0f;
-#pragma unroll
-                for (uint32_t i = 0; i < (uint32_t)NI; i++)
-                    if ((has_data >> i) & 1u) {
-                        ptx::tmem_ld_cols<CH>(acc + i * Cfg::acc_stride + c0, v);
-                        ptx::tc_wait_ld();
-#pragma unroll
-                        for (int u = 0; u < CH; u++) f[u] += __uint_as_float(v[u]);
-                    }
-                if (seg.out_kind == kOutDirect) {
-#pragma unroll
-                    for (int u = 0; u < CH; u++) f[u] = f[u] * row_scale + row_bias;
-                    store_columns(p.out, (int)p.activation, f, n0, p.N, row, lane);
-                } else if (seg.out_kind == kOutSplitPartial) {
-                    float* dst = p.workspace + ((size_t)seg.out_index * p.N + n0) * p.M + row;
-#pragma unroll
-                    for (int u = 0; u < CH; u++)
-                        if (n0 + u < p.N) dst[(size_t)u * p.M] = f[u] * row_scale;
-                } else if (seg.out_kind == kOutClusterPart) {   // into the ring, which is idle: this is the CTA's last segment
-#pragma unroll
-                    for (int u = 0; u < CH; u++)
-                        if (n0 + u < p.N) ptx::sts_f32(ring + ((c0 + u) * kTileM + row_in_tile) * 4u, f[u] * row_scale);
-                } else {   // a pair's slot holds the 256 rows of the plan's tile: each CTA its half
-                    constexpr uint32_t kSlotRows = PAIR ? 2u * kTileM : (uint32_t)kTileM;
-                    float* dst = p.workspace + ((size_t)seg.out_index * p.n_width + c0) * kSlotRows + half_id * kTileM + row_in_tile;
-#pragma unroll
-                    for (int u = 0; u < CH; u++)
-                        if (n0 + u < p.N) dst[u * kSlotRows] = f[u] * row_scale;
-                }
-            }
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (PAIR && half_id != 0u) ptx::mbar_arrive_remote_elected(ptx::mapa(acc_peer, 0u));   // tell the issuing CTA
-            else ptx::mbar_arrive_elected(acc_empty);
-            if (threadIdx.x == 0) PROF_STAMP(8);
             nseg++;
         }
         PROF_FLUSH();
@@ -686,8 +700,17 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
             else ptx::mbar_arrive_elected(pending_bar);
             pending_bar = 0;
         };
-        while (ok && plan_next(plan, cta, &iter, &seg)) {
-            const uint32_t nstages = (seg.nkb + KS - 1) / KS;
+        // Wide tiles: these sixteen warps end the segments too (a group every fourth round of 16 columns).  With the four issuing
+        // warps alone the tensor pipe stood still longer between two tiles: a 13B-like block at 150 tokens 45.7 -> 42.6 us, 70B at
+        // 512 743 -> 730, at 64 197.4 -> 194.5.  A group does it after its first visit of the NEXT segment (whose position only
+        // needs this segment's MMAs to be done), so that the issuing warps find stored slots the moment the accumulators
+        // are free.  Up to 32 columns there are one or two rounds and the unpacking must not wait for them: 13B FP5 layers at 16
+        // tokens 58.6 us with the issuing warps, 62.3 with these.
+        uint32_t last_tile = 0, last_index = 0, last_flags = 0;   // flags: issuers with a sum, out_kind << 4, parity << 8
+        bool pending = false;
+        for (uint32_t nseg = 0;; nseg++) {
+            const bool more = ok && plan_next(plan, cta, &iter, &seg);
+            const uint32_t nstages = more ? (seg.nkb + KS - 1) / KS : 0u;
             uint32_t t = (cls + ST - (j0 % ST)) % ST;     // this group's first stage of the segment
             ptx::RingPos<R> rp;
             rp.set(j0 + t);
@@ -696,53 +719,69 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
                 ap.set((j0 + t) * PPS + group % PPS);
                 slot = ap.idx; slot_lap = ap.lap; slot_primed = 1;
             }
-            for (; t < nstages; t += ST) {
-                if (!PROF_WAIT(0, ptx::mbar_wait_warp(w_full + 8 * rp.idx, rp.lap, abort_word, kErrStageFull, Cfg::poll_unpack))) { ok = false; break; }
-                if (warp == kFirstDequantWarp && lane == 0 && j0 == 0 && t == cls) PROF_STAMP(4);
-                PROF_COUNT(6)
-                if (q == 0) PROF_TRACE(5, j0 + t);
-                const uint32_t raw = lane_base + rp.idx * Cfg::w_stride;   // shared-space byte address of this lane's words
-                load_words(raw, 0);
-                const uint32_t a_addr = a_lane + slot * Cfg::slot_cols;
+            while (ok && (t < nstages || pending)) {
+                if (!Cfg::unpack_ends || t < nstages) {
+                    if (!PROF_WAIT(0, ptx::mbar_wait_warp(w_full + 8 * rp.idx, rp.lap, abort_word, kErrStageFull, Cfg::poll_unpack))) { ok = false; break; }
+                    if (warp == kFirstDequantWarp && lane == 0 && j0 == 0 && t == cls) PROF_STAMP(4);
+                    PROF_COUNT(6)
+                    if (q == 0) PROF_TRACE(5, j0 + t);
+                    const uint32_t raw = lane_base + rp.idx * Cfg::w_stride;   // shared-space byte address of this lane's words
+                    load_words(raw, 0);
+                    const uint32_t a_addr = a_lane + slot * Cfg::slot_cols;
 #pragma unroll
-                for (int b = 0; b < KPW; b++) {
-                    PROF_BEGIN(t_math)
-                    uint32_t v[2][16];
+                    for (int b = 0; b < KPW; b++) {
+                        PROF_BEGIN(t_math)
+                        uint32_t v[2][16];
 #pragma unroll
-                    for (int jj = 0; jj < 4; jj++) {
-                        uint32_t pat[8];
-                        if constexpr (kShortUnpack) unpack16_mul<E_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], km, pat);
-                        else unpack16_generic<E_BITS, M_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], h, pat);
+                        for (int jj = 0; jj < 4; jj++) {
+                            uint32_t pat[8];
+                            if constexpr (kShortUnpack) unpack16_mul<E_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], km, pat);
+                            else unpack16_generic<E_BITS, M_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], h, pat);
 #pragma unroll
-                        for (int kk = 0; kk < 2; kk++)
+                            for (int kk = 0; kk < 2; kk++)
 #pragma unroll
-                            for (int i = 0; i < 4; i++) v[kk][4 * jj + i] = pat[4 * kk + i];
+                                for (int i = 0; i < 4; i++) v[kk][4 * jj + i] = pat[4 * kk + i];
+                        }
+                        PROF_END(1, t_math)
+                        if (b + 1 < KPW) {
+                            load_words(raw, b + 1);
+                        } else {
+                            __syncwarp();
+                            ptx::mbar_arrive_elected(w_empty + 8 * rp.idx);   // the weights can be refilled
+                        }
+                        if (b == 0) {
+                            if (!PROF_WAIT(2, ptx::mbar_wait_warp(a_empty + 8 * slot, slot_lap ^ 1u, abort_word, kErrAEmpty, Cfg::poll_unpack))) { ok = false; break; }
+                            ptx::tc_fence_after_sync();
+                            if (q == 0) PROF_TRACE(6, j0 + t);
+                        }
+                        ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock, v[0]);
+                        ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock + (16u << 16), v[1]);
                     }
-                    PROF_END(1, t_math)
-                    if (b + 1 < KPW) {
-                        load_words(raw, b + 1);
-                    } else {
-                        __syncwarp();
-                        ptx::mbar_arrive_elected(w_empty + 8 * rp.idx);   // the weights can be refilled
+                    if (!ok) break;
+                    {
+                        const uint32_t mine = Cfg::unified ? b_full : a_full, peers = Cfg::unified ? b_full : a_peer;
+                        pending_bar = (PAIR && half_id != 0u) ? ptx::mapa(peers + 8 * slot, 0u) : mine + 8 * slot;
                     }
-                    if (b == 0) {
-                        if (!PROF_WAIT(2, ptx::mbar_wait_warp(a_empty + 8 * slot, slot_lap ^ 1u, abort_word, kErrAEmpty, Cfg::poll_unpack))) { ok = false; break; }
-                        ptx::tc_fence_after_sync();
-                        if (q == 0) PROF_TRACE(6, j0 + t);
-                    }
-                    ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock, v[0]);
-                    ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock + (16u << 16), v[1]);
+                    hand_over();
+                    if (q == 0) PROF_TRACE(7, j0 + t);
+                    slot += kDequantGroups;
+                    if (slot >= (uint32_t)SA) { slot -= SA; slot_lap ^= 1u; }
+                    rp.advance(ST);
+                    t += ST;
                 }
-                if (!ok) break;
-                {
-                    const uint32_t mine = Cfg::unified ? b_full : a_full, peers = Cfg::unified ? b_full : a_peer;
-                    pending_bar = (PAIR && half_id != 0u) ? ptx::mapa(peers + 8 * slot, 0u) : mine + 8 * slot;
+                if constexpr (Cfg::unpack_ends) {
+                    if (pending && !end_segment(last_tile, (last_flags >> 4) & 15u, last_index, last_flags & 15u, last_flags >> 8, group,
+                                                kDequantGroups))
+                        ok = false;
+                    pending = false;
                 }
-                hand_over();
-                if (q == 0) PROF_TRACE(7, j0 + t);
-                slot += kDequantGroups;
-                if (slot >= (uint32_t)SA) { slot -= SA; slot_lap ^= 1u; }
-                rp.advance(ST);
+            }
+            if (!ok || !more) break;
+            if constexpr (Cfg::unpack_ends) {
+                last_tile = seg.tile;
+                last_index = seg.out_index;
+                last_flags = issuers_with_sum(j0, seg.nkb, nstages) | seg.out_kind << 4 | (nseg & 1u) << 8;
+                pending = true;
             }
             j0 += nstages;
         }

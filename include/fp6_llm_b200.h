@@ -33,9 +33,11 @@ const char* fp6b200_error_string(int code);
  * The linear layer on device buffers, asynchronous on `stream` (a cudaStream_t).
  * Stands in for fp_eXmY_linear_kernel (fp6_llm/csrc/fp6_linear.cuh:20-32; with e_bits=3, m_bits=2
  * also for fp6_linear_kernel, :8-18).  `workspace` holds split_k*M*N floats and is only touched
- * when split_k > 1.  split_k == 0 lets the library decompose the work itself (whole waves of output tiles,
- * then the K blocks of the remaining tiles dealt out evenly over the SMs and summed by a fix-up kernel);
+ * when split_k > 1.  split_k == 0 lets the library decompose the work itself (whole output tiles, tiles
+ * shared by a cluster of SMs, or the K blocks of the remaining tiles dealt out evenly and summed by a fix-up kernel);
  * size the workspace with fp6b200_workspace_bytes(M, N, K, 0) in that case.
+ * split_k >= 1 is taken as the offer of that workspace: the library's own decomposition runs wherever it needs no
+ * more (split_k == 1: none), the split as asked otherwise.
  * Unsupported shapes/formats return cudaErrorInvalidValue instead of asserting or exiting.
  */
 int fp6b200_linear(int e_bits, int m_bits, void* stream, const void* weight_packed, const void* scales,
