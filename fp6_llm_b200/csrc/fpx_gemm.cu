@@ -27,8 +27,8 @@
 //               index comes through a shuffle, so addresses and descriptors stay warp-uniform, and a round of four
 //               MMAs and a commit costs ~64 cycles where a branch taken by one lane alone pays ~230, plus ~200 for
 //               every barrier wait whose result it consumes (the copy producers issue the same way).  At the end
-//               of a segment the same four warps (one per tensor-memory lane quadrant) read the accumulators
-//               with tcgen05.ld, add them, multiply by 2^bias * scale[row] in fp32 (the per-row scale is
+//               of a segment the same four warps (narrow tiles) or the sixteen unpack warps read the accumulators (one
+//               warp per tensor-memory lane quadrant) with tcgen05.ld, add them, multiply by 2^bias * scale[row] in fp32 (the per-row scale is
 //               applied here, once per output, not once per weight), add the bias, apply the fused activation and
 //               store fp16 output - to this GPU's buffer or to every rank's - or fp32 partials.
 //
@@ -706,84 +706,95 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         // needs this segment's MMAs to be done), so that the issuing warps find stored slots the moment the accumulators
         // are free.  Up to 32 columns there are one or two rounds and the unpacking must not wait for them: 13B FP5 layers at 16
         // tokens 58.6 us with the issuing warps, 62.3 with these.
-        uint32_t last_tile = 0, last_index = 0, last_flags = 0;   // flags: issuers with a sum, out_kind << 4, parity << 8
-        bool pending = false;
-        for (uint32_t nseg = 0;; nseg++) {
-            const bool more = ok && plan_next(plan, cta, &iter, &seg);
-            const uint32_t nstages = more ? (seg.nkb + KS - 1) / KS : 0u;
-            uint32_t t = (cls + ST - (j0 % ST)) % ST;     // this group's first stage of the segment
-            ptx::RingPos<R> rp;
+        // one visit: the position of running stage `at` (false: a wait gave up)
+        auto visit = [&](ptx::RingPos<R>& rp, uint32_t at) -> bool {
+            if (!PROF_WAIT(0, ptx::mbar_wait_warp(w_full + 8 * rp.idx, rp.lap, abort_word, kErrStageFull, Cfg::poll_unpack))) return false;
+            if (warp == kFirstDequantWarp && lane == 0 && at == cls) PROF_STAMP(4);
+            PROF_COUNT(6)
+            if (q == 0) PROF_TRACE(5, at);
+            const uint32_t raw = lane_base + rp.idx * Cfg::w_stride;   // shared-space byte address of this lane's words
+            load_words(raw, 0);
+            const uint32_t a_addr = a_lane + slot * Cfg::slot_cols;
+#pragma unroll
+            for (int b = 0; b < KPW; b++) {
+                PROF_BEGIN(t_math)
+                uint32_t v[2][16];
+#pragma unroll
+                for (int jj = 0; jj < 4; jj++) {
+                    uint32_t pat[8];
+                    if constexpr (kShortUnpack) unpack16_mul<E_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], km, pat);
+                    else unpack16_generic<E_BITS, M_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], h, pat);
+#pragma unroll
+                    for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) v[kk][4 * jj + i] = pat[4 * kk + i];
+                }
+                PROF_END(1, t_math)
+                if (b + 1 < KPW) {
+                    load_words(raw, b + 1);
+                } else {
+                    __syncwarp();
+                    ptx::mbar_arrive_elected(w_empty + 8 * rp.idx);   // the weights can be refilled
+                }
+                if (b == 0) {
+                    if (!PROF_WAIT(2, ptx::mbar_wait_warp(a_empty + 8 * slot, slot_lap ^ 1u, abort_word, kErrAEmpty, Cfg::poll_unpack))) return false;
+                    ptx::tc_fence_after_sync();
+                    if (q == 0) PROF_TRACE(6, at);
+                }
+                ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock, v[0]);
+                ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock + (16u << 16), v[1]);
+            }
+            {
+                const uint32_t mine = Cfg::unified ? b_full : a_full, peers = Cfg::unified ? b_full : a_peer;
+                pending_bar = (PAIR && half_id != 0u) ? ptx::mapa(peers + 8 * slot, 0u) : mine + 8 * slot;
+            }
+            hand_over();
+            if (q == 0) PROF_TRACE(7, at);
+            slot += kDequantGroups;
+            if (slot >= (uint32_t)SA) { slot -= SA; slot_lap ^= 1u; }
+            rp.advance(ST);
+            return true;
+        };
+        auto first_visit = [&](ptx::RingPos<R>& rp, uint32_t nstages) -> uint32_t {   // this group's first stage of the segment
+            const uint32_t t = (cls + ST - (j0 % ST)) % ST;
             rp.set(j0 + t);
             if (!slot_primed && t < nstages) {            // the group's first position of all: p = (j0 + t) * PPS + group % PPS
                 ptx::RingPos<SA> ap;
                 ap.set((j0 + t) * PPS + group % PPS);
                 slot = ap.idx; slot_lap = ap.lap; slot_primed = 1;
             }
-            while (ok && (t < nstages || pending)) {
-                if (!Cfg::unpack_ends || t < nstages) {
-                    if (!PROF_WAIT(0, ptx::mbar_wait_warp(w_full + 8 * rp.idx, rp.lap, abort_word, kErrStageFull, Cfg::poll_unpack))) { ok = false; break; }
-                    if (warp == kFirstDequantWarp && lane == 0 && j0 == 0 && t == cls) PROF_STAMP(4);
-                    PROF_COUNT(6)
-                    if (q == 0) PROF_TRACE(5, j0 + t);
-                    const uint32_t raw = lane_base + rp.idx * Cfg::w_stride;   // shared-space byte address of this lane's words
-                    load_words(raw, 0);
-                    const uint32_t a_addr = a_lane + slot * Cfg::slot_cols;
-#pragma unroll
-                    for (int b = 0; b < KPW; b++) {
-                        PROF_BEGIN(t_math)
-                        uint32_t v[2][16];
-#pragma unroll
-                        for (int jj = 0; jj < 4; jj++) {
-                            uint32_t pat[8];
-                            if constexpr (kShortUnpack) unpack16_mul<E_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], km, pat);
-                            else unpack16_generic<E_BITS, M_BITS>(w4[jj][0], w4[jj][1], w2[jj], w1[jj], h, pat);
-#pragma unroll
-                            for (int kk = 0; kk < 2; kk++)
-#pragma unroll
-                                for (int i = 0; i < 4; i++) v[kk][4 * jj + i] = pat[4 * kk + i];
-                        }
-                        PROF_END(1, t_math)
-                        if (b + 1 < KPW) {
-                            load_words(raw, b + 1);
-                        } else {
-                            __syncwarp();
-                            ptx::mbar_arrive_elected(w_empty + 8 * rp.idx);   // the weights can be refilled
-                        }
-                        if (b == 0) {
-                            if (!PROF_WAIT(2, ptx::mbar_wait_warp(a_empty + 8 * slot, slot_lap ^ 1u, abort_word, kErrAEmpty, Cfg::poll_unpack))) { ok = false; break; }
-                            ptx::tc_fence_after_sync();
-                            if (q == 0) PROF_TRACE(6, j0 + t);
-                        }
-                        ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock, v[0]);
-                        ptx::tmem_st_16x128b_x8(a_addr + b * kAColsPerKBlock + (16u << 16), v[1]);
-                    }
-                    if (!ok) break;
-                    {
-                        const uint32_t mine = Cfg::unified ? b_full : a_full, peers = Cfg::unified ? b_full : a_peer;
-                        pending_bar = (PAIR && half_id != 0u) ? ptx::mapa(peers + 8 * slot, 0u) : mine + 8 * slot;
-                    }
-                    hand_over();
-                    if (q == 0) PROF_TRACE(7, j0 + t);
-                    slot += kDequantGroups;
-                    if (slot >= (uint32_t)SA) { slot -= SA; slot_lap ^= 1u; }
-                    rp.advance(ST);
+            return t;
+        };
+        if constexpr (!Cfg::unpack_ends) {
+            while (ok && plan_next(plan, cta, &iter, &seg)) {
+                const uint32_t nstages = (seg.nkb + KS - 1) / KS;
+                ptx::RingPos<R> rp;
+                for (uint32_t t = first_visit(rp, nstages); t < nstages; t += ST)
+                    if (!visit(rp, j0 + t)) { ok = false; break; }
+                j0 += nstages;
+            }
+        } else {
+            uint32_t last_tile = 0, last_index = 0, last_flags = 0;   // flags: issuers with a sum, out_kind << 4, parity << 8
+            bool pending = false;
+            for (uint32_t nseg = 0;; nseg++) {
+                const bool more = plan_next(plan, cta, &iter, &seg);
+                const uint32_t nstages = more ? (seg.nkb + KS - 1) / KS : 0u;
+                ptx::RingPos<R> rp;
+                uint32_t t = first_visit(rp, nstages);
+                while (ok && (t < nstages || pending)) {
+                    if (t < nstages) ok = visit(rp, j0 + t);
                     t += ST;
-                }
-                if constexpr (Cfg::unpack_ends) {
-                    if (pending && !end_segment(last_tile, (last_flags >> 4) & 15u, last_index, last_flags & 15u, last_flags >> 8, group,
-                                                kDequantGroups))
-                        ok = false;
+                    if (ok && pending)
+                        ok = end_segment(last_tile, (last_flags >> 4) & 15u, last_index, last_flags & 15u, last_flags >> 8, group, kDequantGroups);
                     pending = false;
                 }
-            }
-            if (!ok || !more) break;
-            if constexpr (Cfg::unpack_ends) {
+                if (!ok || !more) break;
                 last_tile = seg.tile;
                 last_index = seg.out_index;
                 last_flags = issuers_with_sum(j0, seg.nkb, nstages) | seg.out_kind << 4 | (nseg & 1u) << 8;
                 pending = true;
+                j0 += nstages;
             }
-            j0 += nstages;
         }
         PROF_FLUSH();
     }
