@@ -19,6 +19,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <exception>
+#include <vector>
 
 #include "../../include/fp6_llm_b200.h"
 
@@ -176,10 +177,57 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
+// a contiguous fp16 CPU tensor
+const at::Tensor* plain_host(PyObject* o) {
+    if (!THPVariable_CheckExact(o)) return nullptr;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    if (!t.defined() || t.scalar_type() != at::kHalf || !t.is_cpu() || t.layout() != at::kStrided || t.key_set().has_any(kWrapped) ||
+        !t.is_contiguous())
+        return nullptr;
+    return &t;
+}
+
+// host_batch([(e, m, act_host, packed, scales, out_host, split_k[, tiles or None]), ...]) -> True.  The first copy of a batch can
+// start only when all its calls are laid out: in Python that took longer than the copy.
+PyObject* host_batch(PyObject*, PyObject* calls) {
+    HANDLE_TH_ERRORS
+    if (!PyList_CheckExact(calls) || PyList_GET_SIZE(calls) < 1 || PyList_GET_SIZE(calls) > 4096) return not_mine();
+    std::vector<fp6b200_host_call> batch((size_t)PyList_GET_SIZE(calls));
+    int device = -1;
+    for (size_t i = 0; i < batch.size(); i++) {
+        PyObject* c = PyList_GET_ITEM(calls, (Py_ssize_t)i);
+        if (!PyTuple_CheckExact(c) || PyTuple_GET_SIZE(c) < 7 || PyTuple_GET_SIZE(c) > 8) return not_mine();
+        long e, m, split;
+        if (!whole(PyTuple_GET_ITEM(c, 0), &e) || !whole(PyTuple_GET_ITEM(c, 1), &m) || !whole(PyTuple_GET_ITEM(c, 6), &split)) return not_mine();
+        if (e < 0 || e > 7 || m < 0 || m > 7 || split < 0 || split > 65535 || !fp6b200_native_supported((int)e, (int)m, 256, 1, 64)) return not_mine();
+        const at::Tensor* packed = plain(PyTuple_GET_ITEM(c, 3), at::kInt, device);
+        if (!packed || packed->dim() != 2) return not_mine();
+        device = packed->get_device();
+        const at::Tensor* scales = plain(PyTuple_GET_ITEM(c, 4), at::kHalf, device);
+        const at::Tensor *act = plain_host(PyTuple_GET_ITEM(c, 2)), *out = plain_host(PyTuple_GET_ITEM(c, 5)), *tiles = nullptr;
+        if (!scales || !act || !out || act->dim() != 2 || out->dim() != 2) return not_mine();
+        if (PyTuple_GET_SIZE(c) == 8 && PyTuple_GET_ITEM(c, 7) != Py_None && !(tiles = plain(PyTuple_GET_ITEM(c, 7), at::kByte, device)))
+            return not_mine();
+        const int64_t tokens = act->size(0), ic = act->size(1), oc = packed->size(0);
+        if (packed->size(1) * 32 != ic * (1 + e + m) || scales->numel() != oc || out->size(0) != tokens || out->size(1) != oc) return not_mine();
+        batch[i] = {(int)e, (int)m, packed->data_ptr(), scales->data_ptr(), act->data_ptr(), out->data_ptr(), (size_t)oc, (size_t)tokens,
+                    (size_t)ic, (int)split, tiles ? tiles->data_ptr() : nullptr};
+    }
+    const c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, (c10::DeviceIndex)device));
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = fp6b200_linear_host_io_batch(batch.data(), (int)batch.size());
+    Py_END_ALLOW_THREADS
+    if (rc != 0) return fail("fp6b200_linear_host_io_batch", rc);
+    Py_RETURN_TRUE;
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear)), METH_FASTCALL, nullptr},
     {"native", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(native)), METH_FASTCALL, nullptr},
     {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(layer)), METH_FASTCALL, nullptr},
+    {"host_batch", host_batch, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "fp6_b200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -387,6 +387,8 @@ def linear_forward_host_batch(calls) -> None:
     calls = list(calls)
     if not calls:
         return
+    if _native.host().host_batch(calls) is True:
+        return
     arr = (_native.HostCall * len(calls))()
     dev = calls[0][3].device
     for i, call in enumerate(calls):

@@ -24,6 +24,7 @@ def test_declines_what_is_not_a_plain_cuda_call(host):
     assert host.linear(3.0, 2, x, w, s, 0, None, 0) is NotImplemented
     assert host.linear(3, 2, x, w, s, 2 ** 70, None, 0) is NotImplemented
     assert host.linear(3, 2, x) is NotImplemented and host.layer() is NotImplemented
+    assert host.host_batch([]) is NotImplemented and host.host_batch([(3, 2, x, w, s, x, 0)]) is NotImplemented
 
 
 def _layer(oc=512, ic=256, e=3, m=2, bias=True, cls=None):
@@ -36,7 +37,7 @@ def _layer(oc=512, ic=256, e=3, m=2, bias=True, cls=None):
 
 class _Declining:
     """Stands in for the binding so that the Python form runs."""
-    linear = native = layer = staticmethod(lambda *a: NotImplemented)
+    linear = native = layer = host_batch = staticmethod(lambda *a: NotImplemented)
 
 
 @pytest.mark.gpu
@@ -62,6 +63,36 @@ def test_same_as_the_python_form(host, monkeypatch, e, m, batch):
                     want = [layer(t) for t in forms] + [c() for c in calls]
                 for a, b in zip(got, want):
                     assert a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype and torch.equal(a, b)
+    assert f.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_host_batch_same_as_the_python_form(host, monkeypatch):
+    layers = [_layer(512, 256, bias=False).enable_native(), _layer(1280, 1088, 2, 2, bias=False)]
+    def batch(native):
+        calls = []
+        for i, layer in enumerate(layers * 3):
+            act = torch.randn(1 + 20 * i, layer.in_features, generator=torch.Generator().manual_seed(i)).half().pin_memory()
+            out = torch.empty(act.shape[0], layer.out_features, dtype=torch.float16, pin_memory=True)
+            call = (layer.e_bits, layer.m_bits, act, layer.weight, layer.scales, out, 0)
+            calls.append(call + (layer._buffers.get("weight_native"),) if native else call)
+        return calls
+    for native in (False, True):
+        got, want = batch(native), batch(native)
+        assert host.host_batch(list(got)) is True
+        with monkeypatch.context() as mp:
+            mp.setattr(_native, "_host", _Declining)
+            f.linear_forward_host_batch(want)
+        assert all(torch.equal(a[5], b[5]) for a, b in zip(got, want))
+    good = batch(False)[0]
+    for at, bad in ((2, good[2].float()), (2, good[2].cuda()), (2, good[2][:, :64]), (3, good[3][:256]), (5, good[5][:, :256]),
+                    (5, good[5].cuda()), (0, 7)):
+        call = good[:at] + (bad,) + good[at + 1:]
+        assert host.host_batch([call]) is NotImplemented
+        with pytest.raises(ValueError):
+            f.linear_forward_host_batch([call])
+    with pytest.raises(RuntimeError, match="host_io_batch failed"):   # no tokens: refused by the library, as before
+        f.linear_forward_host_batch([good[:2] + (good[2][:0],) + good[3:5] + (good[5][:0],) + good[6:]])
     assert f.device_status() == 0
 
 
