@@ -152,3 +152,54 @@ def test_streams_threads_and_graphs(host):
         t.join()
     torch.cuda.synchronize()
     assert not wrong and all(torch.equal(a, b) for a, b in zip(captured, want)) and f.device_status() == 0
+
+
+def _replaced(layer, how):
+    """The layer with its bias outside the buffers: as a Parameter, as a plain attribute, or as a property of a subclass."""
+    bias = layer.bias
+    if how == "parameter":
+        layer.bias = torch.nn.Parameter(bias)
+    else:
+        del layer.bias
+        if how == "attribute":
+            object.__setattr__(layer, "bias", bias)
+        else:
+            layer.__class__ = type("Sub", (type(layer),), {"bias": property(lambda self: bias)})
+    assert "bias" not in layer._buffers and torch.equal(layer.bias.detach(), bias)
+    return layer
+
+
+@pytest.mark.parametrize("cls", [f.FPxLinear, f.FPxGateUpLinear])
+@pytest.mark.parametrize("how", ["parameter", "attribute", "property"])
+def test_bias_outside_the_buffers_reaches_the_binding(monkeypatch, cls, how):
+    """A bias that is no buffer any more must not look like no bias: what the binding is given, without a GPU."""
+    seen = []
+
+    class Recorder:
+        layer = staticmethod(lambda *a: seen.append(a) or "taken")
+    monkeypatch.setattr(_native, "_host", Recorder)
+    layer = cls(torch.zeros(256, 12, dtype=torch.int32), torch.ones(256, dtype=torch.float16), torch.arange(256.0))
+    x = torch.zeros(1, 64, dtype=torch.float16)
+    assert layer(x) == "taken" and seen[-1][7] is layer.bias and seen[-1][4] is None
+    tiles = torch.zeros(4, dtype=torch.uint8)
+    layer.weight_native = torch.nn.Parameter(tiles, requires_grad=False)
+    layer = _replaced(layer, how)
+    layer(x)
+    e, m, _, weight, native, scales, split, bias, _ = seen[-1]
+    assert bias is not None and torch.equal(bias.detach(), torch.arange(256.0).half())
+    assert weight is layer.weight and scales is layer.scales and torch.equal(native, tiles) and (e, m, split) == (3, 2, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cls", [f.FPxLinear, f.FPxGateUpLinear])
+@pytest.mark.parametrize("how", ["parameter", "attribute", "property"])
+def test_bias_outside_the_buffers(cls, how):
+    for native in (False, True):
+        for batch in (1, 8, 40):
+            layer = _layer(cls=cls)
+            if native:
+                layer.enable_native()
+            x = torch.randn(batch, 256, device="cuda").half()
+            want = layer(x)
+            assert torch.equal(_replaced(layer, how)(x), want)
+    assert f.device_status() == 0
