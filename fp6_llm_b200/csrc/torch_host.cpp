@@ -210,6 +210,10 @@ PyObject* host_batch(PyObject*, PyObject* calls) {
             return not_mine();
         const int64_t tokens = act->size(0), ic = act->size(1), oc = packed->size(0);
         if (packed->size(1) * 32 != ic * (1 + e + m) || scales->numel() != oc || out->size(0) != tokens || out->size(1) != oc) return not_mine();
+        // tiles that this call would read past the end of
+        if (tiles && split == 0 && fp6b200_native_preferred((int)e, (int)m, oc, tokens, ic) &&
+            (size_t)tiles->numel() < fp6b200_native_weight_bytes(oc, ic))
+            return not_mine();
         batch[i] = {(int)e, (int)m, packed->data_ptr(), scales->data_ptr(), act->data_ptr(), out->data_ptr(), (size_t)oc, (size_t)tokens,
                     (size_t)ic, (int)split, tiles ? tiles->data_ptr() : nullptr};
     }

@@ -405,6 +405,13 @@ def linear_forward_host_batch(calls) -> None:
         OC = packed.shape[0]
         if _in_channels(packed, e, m) != IC or tuple(out.shape) != (B, OC) or not (act.is_contiguous() and out.is_contiguous()):
             raise ValueError("shape mismatch between activations, packed weights and output")
+        if packed.dtype != torch.int32 or not packed.is_contiguous():
+            raise ValueError("packed weights must be a contiguous int32 tensor")
+        if scales.dtype != torch.float16 or not scales.is_contiguous() or scales.numel() < OC:
+            raise ValueError("scales must be a contiguous fp16 tensor with OC elements")
+        if (native is not None and split_k == 0 and native_preferred(e, m, OC, IC, B)
+                and native.numel() < _native.lib().fp6b200_native_weight_bytes(OC, IC)):
+            raise ValueError("native weight tensor is smaller than the layer's tiles")
         arr[i] = _native.HostCall(e, m, packed.data_ptr(), scales.data_ptr(), act.data_ptr(), out.data_ptr(), OC, B, IC, split_k,
                                   native.data_ptr() if native is not None else None)
     with torch.cuda.device(dev):

@@ -203,3 +203,28 @@ def test_bias_outside_the_buffers(cls, how):
             want = layer(x)
             assert torch.equal(_replaced(layer, how)(x), want)
     assert f.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_host_batch_refuses_buffers_it_would_read_past(host):
+    """Nothing here is launched: the host checks raise before."""
+    layer = _layer(512, 256, bias=False).enable_native()
+    other = _layer(256, 256, bias=False).enable_native()
+    act = torch.randn(8, 256).half().pin_memory()
+    out = torch.empty(8, 512, dtype=torch.float16, pin_memory=True)
+    good = (3, 2, act, layer.weight, layer.scales, out, 0, layer.weight_native)
+    wide = torch.stack([layer.scales, layer.scales], 1)[:, 0]
+    for at, bad in ((7, other.weight_native), (7, layer.weight_native[:-1]), (4, layer.scales[:500]), (4, layer.scales.float()), (4, wide),
+                    (3, layer.weight.float()), (3, torch.stack([layer.weight, layer.weight], 2)[:, :, 0])):
+        call = good[:at] + (bad,) + good[at + 1:]
+        assert host.host_batch([call]) is NotImplemented
+        with pytest.raises(ValueError):
+            f.linear_forward_host_batch([call])
+    f.linear_forward_host_batch([good])
+    want = out.clone()
+    f.linear_forward_host_batch([good[:7] + (torch.cat([layer.weight_native, other.weight_native]),)])   # longer than needed: as before
+    assert torch.equal(out, want)
+    many = torch.randn(64, 256).half().pin_memory()   # a batch that does not read the tiles does not mind them
+    wide_out = torch.empty(64, 512, dtype=torch.float16, pin_memory=True)
+    f.linear_forward_host_batch([good[:2] + (many,) + good[3:5] + (wide_out, 0, other.weight_native)])
+    assert torch.equal(wide_out, layer(many.cuda()).cpu()) and f.device_status() == 0
