@@ -11,8 +11,8 @@ import torch
 
 from . import _native
 from .formats import bit_width, check_format, magnitudes
-from .ops import (ACT_NONE, ACT_SILU_MUL, interleave_gate_up, linear_forward_ex, linear_forward_native, native_preferred,
-                  native_repack, native_supported, quantize_prepack_cuda, row_scales_cuda)
+from .ops import (ACT_NONE, ACT_SILU_MUL, interleave_gate_up, is_plain_memory, linear_forward_ex, linear_forward_native,
+                  native_preferred, native_repack, native_supported, quantize_prepack_cuda, row_scales_cuda)
 
 
 def _enable_native(layer) -> None:
@@ -76,8 +76,8 @@ class FPxLinear(torch.nn.Module):
     def row_scales(weight: torch.Tensor, e_bits: int, m_bits: int) -> torch.Tensor:
         """max|w| of each output channel mapped to the format's largest magnitude (28 for e3m2, 7 for e2m2)."""
         top = float(magnitudes(e_bits, m_bits)[-1])
-        if (weight.is_cuda and weight.dtype == torch.float16 and weight.dim() == 2 and weight.is_contiguous() and weight.numel()
-                and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0):
+        if (weight.is_cuda and weight.dtype == torch.float16 and weight.dim() == 2 and is_plain_memory(weight) and weight.is_contiguous()
+                and weight.numel() and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0):
             return row_scales_cuda(weight, top)
         return (weight.float().abs().amax(dim=1) / top).clamp_min(2.0 ** -24).to(torch.float16)
 

@@ -10,6 +10,8 @@ import ctypes
 import math
 
 import torch
+from torch.overrides import _get_current_function_mode_stack
+from torch.utils._device import DeviceContext
 
 from . import _native
 from .formats import bit_width, check_format
@@ -296,9 +298,25 @@ def quantize_prepack_cuda(weights: torch.Tensor, scales: torch.Tensor, EXPONENT:
     return out
 
 
+def is_plain_memory(t: torch.Tensor) -> bool:
+    """Whether a kernel that reads t's memory may stand in for tensor operations on t: nothing records the operations (autograd
+    in reverse or forward mode, tracing, an active mode) and t is not a wrapper around something else (a tensor subclass, vmap and
+    the other function transforms, a lazily negated view)."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter)
+            and not (t.requires_grad and torch.is_grad_enabled())
+            and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and not t.is_neg() and not torch._is_zerotensor(t)
+            and torch.autograd.forward_ad.unpack_dual(t).tangent is None
+            and torch._C._len_torch_dispatch_stack() == 0
+            and all(isinstance(mode, DeviceContext) for mode in _get_current_function_mode_stack())   # `with torch.device(..)` is none
+            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+
+
 def row_scales_cuda(weights: torch.Tensor, top: float) -> torch.Tensor:
     """fp16 CUDA weights [OC, IC] (contiguous, IC % 8 == 0, 16-byte aligned) -> fp16 [OC]: max|w| of every row divided by
     `top`, at least 2^-24, in one pass over the weights (C: fp6b200_row_scales; no counterpart in the reference)."""
+    if not weights.is_cuda or weights.dtype != torch.float16 or weights.dim() != 2 or not weights.is_contiguous():
+        raise ValueError("expected a contiguous fp16 CUDA tensor [OC, IC]")
     OC, IC = weights.shape
     out = torch.empty(OC, dtype=torch.float16, device=weights.device)
     with torch.cuda.device(weights.device):

@@ -64,3 +64,24 @@ def test_b200_heuristic_is_sane(native_lib):
         assert 1 <= k <= K // 64
     assert heuristic_split_k_b200(57344, 2048, 8192) == 1        # plenty of tiles: no split
     assert heuristic_split_k_b200(4096, 1, 4096) > 1             # 32 tiles on 148 SMs: split
+
+
+def test_row_scales_of_tensors_without_memory():
+    """A wrapper has no address to give to a kernel: its scales stay a tensor expression (no GPU is needed to trace one)."""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from fp6_llm_b200 import FPxLinear
+    from fp6_llm_b200.ops import is_plain_memory, row_scales_cuda
+    with FakeTensorMode():
+        fake = torch.empty(64, 128, dtype=torch.float16, device="cuda")
+    got = FPxLinear.row_scales(fake, 3, 2)
+    assert got.shape == (64,) and got.dtype == torch.float16 and got.device.type == "cuda"
+    w = torch.randn(4, 8).half()
+    assert is_plain_memory(w) and is_plain_memory(torch.nn.Parameter(w, requires_grad=False))
+    assert not is_plain_memory(torch.nn.Parameter(w)) and not is_plain_memory(torch._neg_view(w))
+    with torch.no_grad():
+        assert is_plain_memory(torch.nn.Parameter(w))
+    for bad in (w, fake.float(), fake.t(), fake[0]):
+        with pytest.raises(ValueError):
+            row_scales_cuda(bad, 28.0)

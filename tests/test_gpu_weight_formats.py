@@ -88,3 +88,53 @@ def test_packer_and_dequantisers_at_unit_edges(native_lib, oracle_mod, e, m, row
     assert native_lib.fp6b200_dequant_packed(e, m, None, packed.data_ptr(), sd.data_ptr(), ctypes.c_void_p(store.data_ptr() + 4), rows, cols) == 0
     torch.cuda.synchronize()
     assert same(store[2:2 + rows * cols].view(rows, cols))
+
+
+def _scales_expression(w, e, m):
+    from fp6_llm_b200.formats import magnitudes
+    return (w.float().abs().amax(dim=1) / float(magnitudes(e, m)[-1])).clamp_min(2.0 ** -24).to(torch.float16)
+
+
+def test_row_scales_stay_a_tensor_expression_where_something_watches(native_lib):
+    """Gradients, vmap, forward mode, subclasses and modes see the operations; under no_grad, and inside `with torch.device`, the
+    kernel gives the same values."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from fp6_llm_b200 import FPxLinear
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    w = torch.randn(64, 128, generator=gen, device="cuda").half()
+    want = _scales_expression(w, 3, 2)
+    p = torch.nn.Parameter(w)
+    got = FPxLinear.row_scales(p, 3, 2)
+    ref = _scales_expression(p, 3, 2)
+    assert got.requires_grad and torch.equal(got, want)
+    (g,), (r,) = (torch.autograd.grad(t.float().sum(), p) for t in (got, ref))
+    assert torch.equal(g, r) and g.abs().sum() > 0
+    with torch.no_grad():
+        assert torch.equal(FPxLinear.row_scales(p, 3, 2), want)
+    batched = torch.func.vmap(lambda t: FPxLinear.row_scales(t, 3, 2))(w.reshape(2, 32, 128))
+    assert torch.equal(batched.reshape(-1), want)
+    out, tangent = torch.func.jvp(lambda t: FPxLinear.row_scales(t, 3, 2), (w,), (torch.ones_like(w),))
+    ref, ref_tangent = torch.func.jvp(lambda t: _scales_expression(t, 3, 2), (w,), (torch.ones_like(w),))
+    assert torch.equal(out, want) and torch.equal(tangent, ref_tangent)
+
+    class Counts(TorchDispatchMode):
+        seen = 0
+
+        def __torch_dispatch__(self, fn, types, args=(), kwargs=None):
+            Counts.seen += fn is torch.ops.aten.amax.default
+            return fn(*args, **(kwargs or {}))
+
+    class Calls(TorchFunctionMode):
+        def __torch_function__(self, fn, types, args=(), kwargs=None):
+            Counts.seen += fn is torch.Tensor.amax
+            return fn(*args, **(kwargs or {}))
+
+    for mode in (Counts, Calls):
+        Counts.seen = 0
+        with mode():
+            assert torch.equal(FPxLinear.row_scales(w, 3, 2), want)
+        assert Counts.seen == 1
+    with torch.device("cuda"):
+        assert torch.equal(FPxLinear.row_scales(w, 3, 2), want)
+    assert torch.equal(FPxLinear.row_scales(torch._neg_view(w), 3, 2), want)
