@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 
 import torch
 from torch.overrides import _get_current_function_mode_stack
@@ -110,6 +111,8 @@ def _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, acti
         raise ValueError("scales must have OC elements")
     if splitK < 0:
         raise ValueError("splitK must be >= 0")
+    if operator.index(splitK) > 65535:   # the library's limit: refused although the split itself is the library's choice
+        _native.check(1, "fp6b200_linear")
     if activation not in (ACT_NONE, ACT_SILU_MUL):
         raise ValueError("activation must be ACT_NONE or ACT_SILU_MUL")
     if bias is not None and (bias.dtype != torch.float16 or bias.numel() != OC or bias.device != _in_feats.device

@@ -228,3 +228,22 @@ def test_host_batch_refuses_buffers_it_would_read_past(host):
     wide_out = torch.empty(64, 512, dtype=torch.float16, pin_memory=True)
     f.linear_forward_host_batch([good[:2] + (many,) + good[3:5] + (wide_out, 0, other.weight_native)])
     assert torch.equal(wide_out, layer(many.cuda()).cpu()) and f.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_splits_the_library_refuses_stay_refused(host):
+    """How K is split is the library's choice, but a splitK it would not take is an error all the same."""
+    layer = _layer()
+    x = torch.randn(4, 256, device="cuda").half()
+    want = f.linear_forward_eXmY_cuda(3, 2, x, layer.weight, layer.scales, 1)
+    for ok in (0, 3, 65535, True):
+        assert torch.equal(f.linear_forward_eXmY_cuda(3, 2, x, layer.weight, layer.scales, ok), want)
+    for bad in (65536, 2 ** 40):
+        with pytest.raises(RuntimeError, match="fp6b200_linear failed: CUDA error 1"):
+            f.linear_forward_eXmY_cuda(3, 2, x, layer.weight, layer.scales, bad)
+        with pytest.raises(RuntimeError, match="fp6b200_linear failed"):
+            f.FPxLinear(layer.weight, layer.scales, split_k=bad)(x)
+    for bad in (1.0, 2.5):
+        with pytest.raises(TypeError):
+            f.linear_forward_eXmY_cuda(3, 2, x, layer.weight, layer.scales, bad)
+    assert f.device_status() == 0
