@@ -1366,7 +1366,9 @@ cudaError_t launch_gemm(int e_bits, int m_bits, cudaStream_t stream, const void*
 
     const int width = pair ? n_tile : tile_width(N);
     if (!workspace && scratch && plan.mode == kStreamK && plan_rem_tiles(plan)) {
-        workspace = static_cast<float*>(scratch->get(scratch->context, gemm_auto_workspace_bytes(N)));
+        // what this plan writes: two slots of rows x tile width per CTA (gemm_auto_workspace_bytes is the bound over all plans)
+        const size_t slot = (size_t)(pair ? 2 * kTileM : kTileM) * width * sizeof(float);
+        workspace = static_cast<float*>(scratch->get(scratch->context, 2 * (size_t)plan.grid * slot));
         if (!workspace) return cudaErrorMemoryAllocation;
         if (reinterpret_cast<uintptr_t>(workspace) & 15) return cudaErrorMisalignedAddress;
     }

@@ -57,16 +57,21 @@ struct Call {
     const at::Tensor *x = nullptr, *weight = nullptr, *native = nullptr, *scales = nullptr, *bias = nullptr;
 };
 
-// The workspace of one call, allocated when it is asked for.  Called from C: an exception (out of memory) waits in `failed`.
+// The workspace of one call, allocated when it is asked for.  Called from C: an exception waits in `failed`.
 struct Workspace {
     at::TensorOptions options;
     at::Tensor memory;
     std::exception_ptr failed;
+    bool full = false;   // it was: no memory left
     static void* get(void* self, size_t bytes) noexcept {
         Workspace* w = static_cast<Workspace*>(self);
         try {
             w->memory = at::empty({(int64_t)bytes}, w->options);
             return w->memory.data_ptr();
+        } catch (const c10::OutOfMemoryError&) {
+            w->failed = std::current_exception();
+            w->full = true;
+            return nullptr;
         } catch (...) {
             w->failed = std::current_exception();
             return nullptr;
@@ -105,7 +110,7 @@ PyObject* run(const Call& c, bool last_dim_only) {
     sizes[dim - 1] = c.activation == kSiluMul ? oc / 2 : oc;
     at::Tensor out = at::empty(sizes, at::TensorOptions().device(x.device()).dtype(at::kHalf));
     // The workspace goes back to the allocator when this returns; the stream orders whoever gets it next behind these kernels.
-    Workspace ws{at::TensorOptions().device(x.device()).dtype(at::kByte), {}, nullptr};
+    Workspace ws{at::TensorOptions().device(x.device()).dtype(at::kByte), {}, nullptr, false};
     void* stream = c10::cuda::getCurrentCUDAStream(x.get_device()).stream();
     const void* bias = c.bias ? c.bias->data_ptr() : nullptr;
     void *xp = x.data_ptr(), *op = out.data_ptr(), *sp = c.scales->data_ptr();
@@ -113,8 +118,15 @@ PyObject* run(const Call& c, bool last_dim_only) {
     void* planes = c.native ? Workspace::get(&ws, fp6b200_native_workspace_bytes(batch, ic)) : nullptr;
     int rc = 0;
     Py_BEGIN_ALLOW_THREADS   // a full launch queue blocks
-    if (!c.native) rc = fp6b200_linear_scratch(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, &Workspace::get, &ws, bias, c.activation);
-    else if (planes) rc = fp6b200_linear_native(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, planes, bias, c.activation);
+    if (!c.native) {
+        rc = fp6b200_linear_scratch(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, &Workspace::get, &ws, bias, c.activation);
+        if (ws.full) {   // nothing was launched: the call runs as one that offers no workspace
+            ws.failed = nullptr;
+            rc = fp6b200_linear_ex(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, nullptr, 1, bias, c.activation);
+        }
+    } else if (planes) {
+        rc = fp6b200_linear_native(c.e, c.m, stream, wp, sp, xp, op, oc, batch, ic, planes, bias, c.activation);
+    }
     Py_END_ALLOW_THREADS
     if (ws.failed) std::rethrow_exception(ws.failed);
     if (rc != 0) return fail(c.native ? "fp6b200_linear_native" : "fp6b200_linear", rc);

@@ -74,6 +74,26 @@ def _workspace(device, nbytes: int) -> torch.Tensor:
     return ws
 
 
+class _CallWorkspace:
+    """The workspace of one call, allocated if the library asks for one.  `get` is called from C: what goes wrong waits in
+    `failed`."""
+
+    _TYPE = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)
+
+    def __init__(self, device):
+        self.memory = self.failed = None
+
+        def get(_, nbytes):
+            try:
+                self.memory = torch.empty(nbytes, dtype=torch.uint8, device=device)
+                return self.memory.data_ptr()
+            except Exception as e:   # noqa: BLE001
+                self.failed = e
+                return None
+        self._callback = self._TYPE(get)
+        self.get = ctypes.cast(self._callback, ctypes.c_void_p)
+
+
 def _in_channels(weights: torch.Tensor, e_bits: int, m_bits: int) -> int:
     bw = bit_width(e_bits, m_bits)
     if weights.dim() != 2 or (weights.shape[1] * 32) % bw:
@@ -121,12 +141,17 @@ def _linear(EXPONENT, MANTISSA, _in_feats, _weights, _scales, splitK, bias, acti
     dev = _in_feats.device
     L = _native.lib()
     with torch.cuda.device(dev):
-        # one workspace per call, as in the reference (fp6_llm/csrc/fp6_linear.cu:185-187)
-        # and with it the library's own split of K, whatever the caller names
-        ws = torch.empty(L.fp6b200_workspace_bytes(OC, B, IC, 0), dtype=torch.uint8, device=dev)
         out = torch.empty((B, OC // 2 if activation == ACT_SILU_MUL else OC), dtype=torch.float16, device=dev)
-        rc = L.fp6b200_linear_ex(EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats),
-                                 _ptr(out), OC, B, IC, _ptr(ws), 0, _ptr(bias) if bias is not None else None, activation)
+        # the workspace belongs to the call, as in the reference (fp6_llm/csrc/fp6_linear.cu:185-187), and comes with the
+        # library's own split of K, whatever the caller names
+        ws = _CallWorkspace(dev)
+        args = (EXPONENT, MANTISSA, _stream_ptr(dev), _ptr(_weights), _ptr(_scales), _ptr(_in_feats), _ptr(out), OC, B, IC)
+        end = (_ptr(bias) if bias is not None else None, activation)
+        rc = L.fp6b200_linear_scratch(*args, ws.get, None, *end)
+        if isinstance(ws.failed, torch.OutOfMemoryError):   # nothing was launched: the call runs as one that offers no workspace
+            rc = L.fp6b200_linear_ex(*args, None, 1, *end)
+        elif ws.failed is not None:
+            raise ws.failed
     _native.check(rc, "fp6b200_linear")
     return out
 

@@ -83,3 +83,56 @@ def test_scratch_is_asked_for_only_when_needed(native_lib):
         if needs:
             assert call(None) == 2   # cudaErrorMemoryAllocation, nothing launched
     assert f.device_status() == 0
+
+
+def test_operators_take_no_more_workspace_than_the_plan_writes(native_lib):
+    """Two slots of 128 rows x the tile's columns per SM, not of the kernel's widest tile."""
+    import ctypes
+    import fp6_llm_b200 as f
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    asked = []
+    get = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t)(lambda ctx, n: asked.append(n))   # has none to give
+    for oc, ic, bs, columns in ((10240, 8192, 4, 16), (10240, 8192, 70, 80), (10240, 8192, 130, 144), (10240, 8192, 200, 208),
+                                (19200, 2048, 130, 144), (19200, 2048, 300, 160), (12288, 8192, 300, 160), (11008, 4096, 140, 144)):
+        packed, s, x, _, plain = _layer(oc, ic, bs, 3, 2)
+        out = torch.empty(bs, oc, dtype=torch.float16, device="cuda")
+        del asked[:]
+        rc = native_lib.fp6b200_linear_scratch(3, 2, torch.cuda.current_stream().cuda_stream, packed.data_ptr(), s.data_ptr(), x.data_ptr(),
+                                               out.data_ptr(), oc, bs, ic, ctypes.cast(get, ctypes.c_void_p), None, None, 0)
+        needs = native_lib.fp6b200_kernel_launches(oc, bs, ic, 0) == 2
+        assert rc == (2 if needs else 0) and len(asked) == int(needs)
+        assert all(0 < n <= 2 * sms * 128 * columns * 4 for n in asked)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        y = f.linear_forward_cuda(x, packed, s, 1)
+        peak = torch.cuda.max_memory_allocated() - before
+        assert peak <= y.numel() * 2 + sum(asked) + (2 << 20) and _rel(y, plain) < REL
+    assert f.device_status() == 0
+
+
+@pytest.mark.parametrize("form", ["native", "python"])
+def test_operators_run_without_a_workspace_when_memory_is_full(native_lib, monkeypatch, form):
+    """A caller with room for the result and no more (as with splitK = 1 and no workspace before the split became the library's
+    choice): the torch allocator's limit stands in for a full GPU."""
+    import fp6_llm_b200 as f
+    from fp6_llm_b200 import _native
+    oc, ic, bs = 10240, 8192, 130
+    packed, s, x, bias, plain = _layer(oc, ic, bs, 3, 2)
+    assert native_lib.fp6b200_kernel_launches(oc, bs, ic, 0) == 2   # wants a workspace
+    if form == "python":
+        monkeypatch.setattr(_native, "_host", type("Declining", (), {"linear": staticmethod(lambda *a: NotImplemented)}))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = torch.empty(bs, oc, dtype=torch.float16, device="cuda")
+    total, rest = torch.cuda.get_device_properties(0).total_memory, []
+    try:
+        torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / total)
+        with pytest.raises(torch.OutOfMemoryError):
+            for _ in range(1000):                                   # what the pool still has in pieces a workspace fits into
+                rest.append(torch.empty(20 << 20, dtype=torch.uint8, device="cuda"))
+        del held                                                    # room for one result
+        y = f.linear_forward_ex(3, 2, x, packed, s, 1, bias)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert _rel(y, plain + bias.double()) < REL and f.device_status() == 0
