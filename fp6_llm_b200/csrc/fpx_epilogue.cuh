@@ -18,13 +18,10 @@
 
 namespace fpx {
 
-// silu(gate) * up in fp32; the reciprocal is the hardware's (1 ulp, subnormal results kept, so that it is 0 only for an
-// infinite denominator): the result is rounded to 11 bits next.
-__device__ __forceinline__ float silu_mul(float gate, float up) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(1.0f + __expf(-gate)));
-    return gate * r * up;
-}
+// silu(gate) * up in fp32, every operation rounded once: 3.29 units of 2^-24 off on average over gates of -30 .. 30, 30.5 at most
+// (the exponential's part).  With the hardware's approximate reciprocal instead of the division it was 3.32 and 31.1, and
+// whole passes ran 1 - 2 % faster (70B block at 64 tokens 189.7 against 193.4 us, at 512 708 against 715): precision counts.
+__device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }
 
 __device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
     const __half2 h = __floats2half2_rn(lo, hi);

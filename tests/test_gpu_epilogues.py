@@ -90,6 +90,24 @@ def test_silu_mul_extremes():
     assert torch.allclose(y.double().cpu(), truth.half().double().expand(bs, -1), rtol=1e-3, atol=6e-8)
 
 
+def test_silu_mul_is_as_exact_as_an_ieee_division(tmp_path, native_lib):
+    """The fp32 arithmetic of the gate/up product, against 64 bits, is no further off than gate / (1 + exp(-gate)) * up with every
+    operation rounded once (a reciprocal in its place has one more rounding, and an error of its own)."""
+    import os
+    import subprocess
+    from fp6_llm_b200 import _native
+    here = os.path.dirname(os.path.abspath(__file__))
+    exe = str(tmp_path / "silu_error")
+    done = subprocess.run([_native._nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-O2", "-std=c++17",
+                           os.path.join(here, "cxx", "silu_error.cu"), "-o", exe], capture_output=True, text=True)
+    assert done.returncode == 0, done.stdout + done.stderr
+    done = subprocess.run([exe], capture_output=True, text=True)
+    assert done.returncode == 0, done.stdout + done.stderr
+    worst, mean, div_worst, div_mean, differ = (float(v) for v in done.stdout.split())
+    assert 0 < div_mean < 4, done.stdout          # units of 2^-24: exp and three roundings
+    assert worst <= div_worst and mean <= div_mean, done.stdout
+
+
 def test_gate_up_module_matches_two_linears():
     """FPxGateUpLinear.from_linears: interleaves, quantises and packs two torch layers; its output equals silu(gate) * up
     computed in fp32 from the dequantised weights, and FPxLinear adds its bias inside the kernel."""
