@@ -1,8 +1,9 @@
-"""Builds and loads libfp6_b200.so (the CUDA kernels behind the C interface in include/fp6_llm_b200.h) and fp6_b200_host.so
-(the layer call on torch tensors, csrc/torch_host.cpp).
+"""Builds and loads libfp6_b200.so (the CUDA kernels behind the C interface in include/fp6_llm_b200.h) and the extension
+fp6_b200_host (the layer call on torch tensors, csrc/torch_host.cpp).
 
 The library is compiled in-tree with nvcc for sm_100a only.  There is no fallback of any kind: if the
-library is missing or fails to load, every operator raises.
+library is missing or fails to load, every operator raises.  The extension only shortens the way to it: it is compiled against one
+torch and one Python, which its file name carries, and without it the operators reach the same kernels through ctypes.
 """
 from __future__ import annotations
 
@@ -12,13 +13,14 @@ import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
+import warnings
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 _ROOT = os.path.dirname(_PKG)
 _CSRC = os.path.join(_PKG, "csrc")
 LIB_DIR = os.path.join(_PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libfp6_b200.so")
-HOST_PATH = os.path.join(LIB_DIR, "fp6_b200_host.so")
 HOST_SOURCE = "torch_host.cpp"
 SOURCES = ("fpx_gemm.cu", "fpx_native.cu", "fpx_prepack.cu", "c_api.cu", "c_api_noalloc.cu")
 HEADERS = ("fpx_codes.cuh", "fpx_epilogue.cuh", "fpx_internal.h", "fpx_layout.h", "ptx_sm100.cuh")
@@ -54,6 +56,12 @@ def _nvcc() -> str:
     return cand
 
 
+def host_path() -> str:
+    """Where the extension for the running torch and Python is: its interface is that of their headers."""
+    import torch
+    return os.path.join(LIB_DIR, f"fp6_b200_host-torch{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
 def _stale(path: str, sources) -> bool:
     if not os.path.exists(path):
         return True
@@ -72,13 +80,11 @@ def _run(what: str, cmd) -> str:
 
 def _build_host() -> None:
     """The Python binding of the layer call: plain C++ against torch's headers, linked to the library beside it."""
-    import sysconfig
-
     import torch
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", HOST_PATH, os.path.join(_CSRC, HOST_SOURCE)]
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", host_path(), os.path.join(_CSRC, HOST_SOURCE)]
     for inc in (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                 os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
         cmd += ["-isystem", inc]
@@ -96,7 +102,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         out = _run("nvcc", cmd + [os.path.join(_CSRC, s) for s in SOURCES])
         if verbose:
             print(out)
-    if force or _stale(HOST_PATH, (HOST_SOURCE,)):
+    if force or _stale(host_path(), (HOST_SOURCE,)):
         _build_host()
     return LIB_PATH
 
@@ -183,20 +189,30 @@ def lib() -> ctypes.CDLL:
     return L
 
 
+class _PythonForm:
+    """Stands in for the extension: every call is left to the Python form of the same operator."""
+    linear = native = layer = host_batch = staticmethod(lambda *args: NotImplemented)
+
+
 _host = None
 
 
 def host():
-    """The native host side of the layer call (csrc/torch_host.cpp).  Raises if it has not been built."""
+    """The native host side of the layer call (csrc/torch_host.cpp); where it has not been built for this torch and Python, or does
+    not load, a warning and a stand-in that declines every call."""
     global _host
     if _host is None:
         lib()
-        if not os.path.exists(HOST_PATH):
-            raise RuntimeError(f"{HOST_PATH} is missing: build it first (fp6_llm_b200.build()); there is no fallback path")
         import torch  # noqa: F401  (its libraries must be loaded first)
-        loader = importlib.machinery.ExtensionFileLoader("fp6_b200_host", HOST_PATH)
-        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fp6_b200_host", HOST_PATH, loader=loader))
-        loader.exec_module(module)
+        path = host_path()
+        try:
+            loader = importlib.machinery.ExtensionFileLoader("fp6_b200_host", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("fp6_b200_host", path, loader=loader))
+            loader.exec_module(module)
+        except ImportError as e:
+            warnings.warn(f"no native host side for the layer calls ({e}): they go through ctypes, 20 - 30 us slower each; "
+                          "fp6_llm_b200.build() compiles it", RuntimeWarning, stacklevel=3)
+            module = _PythonForm
         _host = module
     return _host
 

@@ -27,6 +27,37 @@ def test_declines_what_is_not_a_plain_cuda_call(host):
     assert host.host_batch([]) is NotImplemented and host.host_batch([(3, 2, x, w, s, x, 0)]) is NotImplemented
 
 
+def test_extension_belongs_to_one_torch_and_one_python(native_lib, monkeypatch):
+    """After an upgrade the file of the old version is not the one that is looked for, built or loaded."""
+    import os
+    import sysconfig
+    path = _native.host_path()
+    assert os.path.exists(path) and torch.__version__ in os.path.basename(path) and path.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert not _native._stale(path, (_native.HOST_SOURCE,))
+    monkeypatch.setattr(torch, "__version__", "9.9.9")
+    assert _native.host_path() != path and _native._stale(_native.host_path(), (_native.HOST_SOURCE,))
+
+
+@pytest.mark.parametrize("content", [None, b"no library"])
+def test_operators_do_without_the_extension(native_lib, monkeypatch, tmp_path, content):
+    """A missing or unusable extension is a warning, once, and the Python form of every call."""
+    import warnings
+    path = tmp_path / "fp6_b200_host.so"
+    if content is not None:
+        path.write_bytes(content)
+    monkeypatch.setattr(_native, "host_path", lambda: str(path))
+    monkeypatch.setattr(_native, "_host", None)
+    with pytest.warns(RuntimeWarning, match="no native host side"):
+        stand_in = _native.host()
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")
+        assert _native.host() is stand_in
+    assert stand_in.linear(1) is stand_in.native() is stand_in.layer(1, 2) is stand_in.host_batch([]) is NotImplemented
+    if torch.cuda.is_available():
+        layer, x = _layer(), torch.randn(3, 256, device="cuda").half()
+        assert layer(x).shape == (3, 512) and f.device_status() == 0
+
+
 def _layer(oc=512, ic=256, e=3, m=2, bias=True, cls=None):
     gen = torch.Generator(device="cuda").manual_seed(oc + ic)
     w = torch.randn(oc, ic, generator=gen, device="cuda").half() * 0.02
