@@ -136,3 +136,64 @@ def test_operators_run_without_a_workspace_when_memory_is_full(native_lib, monke
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert _rel(y, plain + bias.double()) < REL and f.device_status() == 0
+
+
+# The caller's own split (splits as partial sums in his workspace, a reduction behind) and waves of whole tiles: more tiles than
+# SMs, a remainder that no cluster takes (two CTAs a tile do not fit, or K is too short to share), and less workspace than two
+# slots per SM.  Splits of 4 + 5 and 3 + 2 + 2 K blocks, one block each, more splits than blocks; one and two token tiles.
+CALLERS_SPLIT = [(28672, 576, 8, 2), (19200, 448, 5, 3), (19200, 448, 1, 12), (19200, 448, 40, 2), (19200, 448, 130, 2),
+                 (9728, 448, 300, 2), (28672, 8192, 8, 2)]
+
+
+@pytest.mark.parametrize("oc,ic,bs,split_k", CALLERS_SPLIT)
+@pytest.mark.parametrize("e,m", [(3, 2), (2, 2)])
+def test_callers_split_runs_as_asked(native_lib, oc, ic, bs, split_k, e, m):
+    import fp6_llm_b200 as f
+    packed, s, x, bias, plain = _layer(oc, ic, bs, e, m)
+    blocks = ic // 64
+    splits = min(split_k, blocks)
+    elems = split_k * oc * bs
+    stream = torch.cuda.current_stream().cuda_stream
+    assert native_lib.fp6b200_kernel_launches(oc, bs, ic, split_k) == 2
+    pre = plain + bias.double()
+    for with_bias, activation, truth in ((False, f.ACT_NONE, plain), (True, f.ACT_NONE, pre),
+                                         (True, f.ACT_SILU_MUL, torch.nn.functional.silu(pre[:, 0::2]) * pre[:, 1::2])):
+        held = torch.full((elems + 4096,), float("nan"), device="cuda")
+        out = torch.empty(bs, oc // 2 if activation else oc, dtype=torch.float16, device="cuda")
+        assert native_lib.fp6b200_linear_ex(e, m, stream, packed.data_ptr(), s.data_ptr(), x.data_ptr(), out.data_ptr(), oc, bs, ic,
+                                            held.data_ptr(), split_k, bias.data_ptr() if with_bias else None, activation) == 0
+        assert _rel(out, truth) < REL
+        # the route: every split left the whole product of its K blocks, in order, and nothing else was written
+        parts = held[:splits * oc * bs].view(splits, bs, oc)
+        assert not parts.isnan().any() and bool(held[splits * oc * bs:].isnan().all())
+        assert _rel(parts.double().sum(0), plain) < 1e-5
+        if activation == f.ACT_NONE and not with_bias and splits < blocks:
+            codes = f.dequant_packed_cuda(e, m, packed, torch.ones_like(s))[:512].double() * s[:512].double()[:, None]
+            k0 = 0
+            for z in range(splits):
+                k1 = k0 + (blocks // splits + (z < blocks % splits)) * 64
+                assert _rel(parts[z, :, :512], x[:, k0:k1].double() @ codes[:, k0:k1].T) < 1e-5
+                k0 = k1
+    plainly = torch.empty(bs, oc, dtype=torch.float16, device="cuda")
+    held = torch.empty(elems, device="cuda")
+    assert native_lib.fp6b200_linear(e, m, stream, packed.data_ptr(), s.data_ptr(), x.data_ptr(), plainly.data_ptr(), oc, bs, ic,
+                                     held.data_ptr(), split_k) == 0
+    assert _rel(plainly, plain) < REL and f.device_status() == 0
+
+
+@pytest.mark.parametrize("oc,ic,bs", [(19200, 448, 1), (19200, 448, 40), (28672, 448, 20), (9728, 448, 300), (37888, 64, 130)])
+def test_waves_of_whole_tiles_without_a_workspace(native_lib, oc, ic, bs):
+    """split_k = 1 with more tiles than SMs and a K too short to share: one kernel, some CTAs with a tile more than others."""
+    import fp6_llm_b200 as f
+    tiles = oc // 128 * ((bs + 255) // 256)
+    assert tiles > torch.cuda.get_device_properties(0).multi_processor_count and ic < 512
+    packed, s, x, bias, plain = _layer(oc, ic, bs, 3, 2)
+    pre = plain + bias.double()
+    stream = torch.cuda.current_stream().cuda_stream
+    assert native_lib.fp6b200_kernel_launches(oc, bs, ic, 1) == 1
+    for activation, truth in ((f.ACT_NONE, pre), (f.ACT_SILU_MUL, torch.nn.functional.silu(pre[:, 0::2]) * pre[:, 1::2])):
+        out = torch.empty(bs, oc // 2 if activation else oc, dtype=torch.float16, device="cuda")
+        assert native_lib.fp6b200_linear_ex(3, 2, stream, packed.data_ptr(), s.data_ptr(), x.data_ptr(), out.data_ptr(), oc, bs, ic, None, 1,
+                                            bias.data_ptr(), activation) == 0
+        assert _rel(out, truth) < REL
+    assert f.device_status() == 0
