@@ -7,8 +7,8 @@
 // two columns), lanes two and four apart do the same with the packed halves, and a lane stores 8 bytes (four rows of one
 // column): plain 12 shuffles + 4 stores, gate/up 14 shuffles + 8 products + 2 stores.  The tensor cores wait meanwhile (the
 // next tile needs the accumulator), so this is main-loop time: a tile of 256 columns with the gate/up product gave up ~17 us
-// beside ~50 us of MMAs.  57344 x 8192 gate/up in a chain of such layers: 1800 -> 1488 us at 2048 tokens, 420 -> 378 us at
-// 512; 22016 x 4096 at 128 tokens 38.6 -> 30.0 us.
+// beside ~50 us of MMAs.  57344 x 8192 gate/up layers in a chain, together with the tile ends on the unpack warps
+// (fpx_gemm.cu): 1763 -> 1540 us at 2048 tokens, 397 -> 335 us at 512, where the same layers without the product take 1440 and 346.
 #pragma once
 #include <cuda_fp16.h>
 #include <stdint.h>

@@ -36,8 +36,10 @@
 // (fpx_native.cu); this kernel is the general one.
 //
 // The kernel is launched programmatically: it starts while the previous kernel of the stream is finishing and every
-// role executes griddepcontrol.wait before it first touches global memory (weights that the caller declared
-// static are requested before that).  Ring depths are multiples of the stride of every role that visits only every
+// role executes griddepcontrol.wait before it first reads or writes global memory.  Two exceptions: weights that the caller
+// declared static are read before that, and of others the first stages are asked into L2 (narrow tiles), which hands
+// nothing to the program: what the previous kernel still writes goes to the same L2 and is what the copies behind the wait
+// find.  Ring depths are multiples of the stride of every role that visits only every
 // n-th position (see Config).
 //
 // Every mbarrier wait is bounded; on a time-out the CTA records a code in a status word, drains its
@@ -511,11 +513,11 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         }
         __syncwarp();
     } else if (warp < kMaxIssuers) {
-        // ------------------------------------------------------------ MMA issue + epilogue
+        // ------------------------------------------------------------ MMA issue (+ the epilogue of narrow tiles)
         // Per segment: the first NI warps issue the MMAs, each converged with one elected lane (issuer i takes the K blocks i, i + NI, ... of every
         // stage, each as soon as its slot of the tensor-memory ring is full, and accumulates them in its own
-        // accumulator); then all four warps, one per tensor-memory lane quadrant, read the accumulators, add them and
-        // store the tile (lane = output channel, column = token).
+        // accumulator).  Up to 32 columns all four warps, one per tensor-memory lane quadrant, then read the accumulators, add
+        // them and store the tile (lane = output channel, column = token); wider tiles end on the unpack warps.
         const uint32_t idesc = p.idesc;
         const uint32_t b_step = PAIR ? Cfg::b_block >> 4 : p.n_width * 8u;   // from one K block's activations to the next, in descriptor units
         // In a pair the first CTA issues for both.  The second CTA's issuing warp has nothing to do in the main loop: its
@@ -702,7 +704,7 @@ fpx_gemm_kernel(const __grid_constant__ CUtensorMap act_map, const __grid_consta
         };
         // Wide tiles: these sixteen warps end the segments too (a group every fourth round of 16 columns).  With the four issuing
         // warps alone the tensor pipe stood still longer between two tiles: a 13B-like block at 150 tokens 45.7 -> 42.6 us, 70B at
-        // 512 743 -> 730, at 64 197.4 -> 194.5.  A group does it after its first visit of the NEXT segment (whose position only
+        // 512 743 -> 730, at 64 197.4 -> 194.5 (one box, both forms in turn; boxes differ by 5 %).  A group does it after its first visit of the NEXT segment (whose position only
         // needs this segment's MMAs to be done), so that the issuing warps find stored slots the moment the accumulators
         // are free.  Up to 32 columns there are one or two rounds and the unpacking must not wait for them: 13B FP5 layers at 16
         // tokens 58.6 us with the issuing warps, 62.3 with these.
@@ -1072,7 +1074,8 @@ int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, const Pl
             const uint64_t waves = tiles / (clusters * c), rem = tiles - waves * clusters * c;
             if (rem > clusters || rem == 0) continue;
             // with waves before it, a size that does not divide the SM groups evenly waits for its SMs to come free together:
-            // 57344 x 8192 at 64 tokens, native path 61.5 us with three, 57.9 with two
+            // 57344 x 8192 on the native path, three against two: 61.5 and 57.9 us at 16 tokens, 108.9 and 102.4 at 64 (the one layer
+            // where the costs would have picked three; five, six and seven go with it unmeasured)
             if (waves && (c & (c - 1))) continue;
             const double cost = phase(kb * (double)waves, (double)(waves * clusters * c) * kb) +
                                 phase((double)((plan.kblocks + c - 1) / c), (double)rem * kb) + costs.reduce + (waves ? costs.segment : 0.0);
@@ -1114,7 +1117,8 @@ cudaError_t launch_one(cudaStream_t stream, const CUtensorMap& map, const Params
         if (dev >= 0 && dev < 64) configured[dev].store(true, std::memory_order_release);
     }
     // Programmatic launch: the CTAs may start, set up and find their work while the previous kernel of the stream is
-    // still finishing; every role waits (griddepcontrol.wait) before it first touches global memory.
+    // still finishing; every role waits (griddepcontrol.wait) before it first reads or writes global memory, static weights and
+    // requests to L2 apart (see the top of the file).
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(PAIR ? 2 * prm.plan.grid : prm.plan.grid);   // a pair of CTAs (a cluster of two) per entry of the plan
     cfg.blockDim = dim3(kThreads);
@@ -1205,7 +1209,7 @@ int max_clusters(int ctas) {
     return found;
 }
 
-static std::atomic<int> g_pair_tiles{0};   // off: measured 0.6 of the single-CTA speed (see Config)
+static std::atomic<int> g_pair_tiles{0};   // off: measured 0.9 of the single-CTA speed (see Config)
 void set_pair_tiles(int on) { g_pair_tiles.store(on < 0 ? 0 : (on > 2 ? 2 : on)); }   // 2: also for layers too small to occupy every pair
 int pair_tiles() { return g_pair_tiles.load(); }
 
@@ -1219,10 +1223,10 @@ static int tile_width(size_t N) {
     return (int)((share + 15) / 16 * 16);
 }
 
-// Whether a call runs as CTA pairs on 256-row tiles (the widest tile only, the library's own decomposition, enough row
-// tiles to occupy the pairs), and its plan: for a pair the plan's row tiles are 256 rows and its "CTAs" are pairs.
 // Microseconds, measured on the layers of 7B and 70B models (4096 x 4096 .. 57344 x 8192, 1 .. 256 tokens) with each
-// decomposition forced in turn; 64-wide K blocks of 128 rows, six bits per weight.  Against the fix-up kernel a cluster's shared
+// decomposition forced in turn; 64-wide K blocks of 128 rows, six bits per weight.  The same figures serve every format: five- and
+// four-bit weights move less and the formats without a short unpack sequence take longer per block, which was not measured
+// apart, so for them the choice is an approximation.  Against the fix-up kernel a cluster's shared
 // memory saves 0.5 us at one token and 4 at 256 (8192 x 8192: 15.2 -> 14.5 us at 16 tokens, 22.9 -> 20.7 at 128, 34.0 -> 30.7 at
 // 256; 8192 x 28672 at 256 tokens 92.2 -> 88.3), and whole tiles beat both while two thirds of the SMs have one (12288 x 4096: 14.6
 // -> 12.2 us at 16 tokens, 22.5 -> 18.3 at 128; with 80 tiles of 148 they lose, 18.6 against 20.4 us).
@@ -1236,6 +1240,8 @@ static PlanCosts plan_costs(size_t N) {
     c.segment = 1.5;
     return c;
 }
+// Whether a call runs as CTA pairs on 256-row tiles (the widest tile only, the library's own decomposition, enough row
+// tiles to occupy the pairs), and its plan: for a pair the plan's row tiles are 256 rows and its "CTAs" are pairs.
 static int plan_call(size_t M, size_t N, size_t K, int split_k, bool has_targets, WorkPlan* plan, bool* pair) {
     const int n_tile = gemm_n_tile(N);
     const size_t n_tiles = gemm_n_tiles(N);

@@ -91,16 +91,7 @@ FPX_HD uint32_t read_code(const uint8_t* row, uint32_t c, int bw) {
 // is [s 0 0 e2 e1 e0 m1 m0] and for E=2,M=2 it is [s 0 0 0 e1 e0 m1 m0]; the low byte is zero.
 // The value is then 2^-(16 - 2^(E-1)) times the FPx value.
 //
-// `hi4` holds in every byte the 4-bit segment of one code (already masked to the low nibble).
-// For e3m2, `s_src` has the sign at bit 7 of every byte and `e_src` has e2 at bit 4 of every byte
-// (other bits arbitrary).  For e2m2, `s_src` has the sign at bit 7 (e_src unused).
-// Returns the four high bytes; out_lo/out_hi expand them into two half2 patterns:
-//   out_lo = (byte1 -> low half, byte3 -> high half), out_hi = (byte0 -> low half, byte2 -> high half).
-FPX_HD uint32_t stitch_e3m2(uint32_t s_src, uint32_t e_src, uint32_t nib) {
-    return (s_src & 0x80808080u) | ((e_src & 0x10101010u) | nib);
-}
-FPX_HD uint32_t stitch_e2m2(uint32_t s_src, uint32_t nib) { return (s_src & 0x80808080u) | nib; }
-
+// Four such high bytes in one word expand into two half2 patterns each:
 FPX_HD uint32_t expand_13(uint32_t y) {   // bytes 3,1 -> high bytes of the two halves
 #if defined(__CUDA_ARCH__)
     return __byte_perm(y, 0u, 0x3414);
@@ -116,44 +107,23 @@ FPX_HD uint32_t expand_02(uint32_t y) {   // bytes 2,0 -> high bytes of the two 
 #endif
 }
 
-// Unpack the 16 codes that one lane owns in two vertically adjacent 16x16 blocks (sub-blocks
-// 2h and 2h+1 of a 64-row block, same 16 columns) into eight half2 bit patterns
+// What is unpacked at a time: the 16 codes that one lane owns in two vertically adjacent 16x16 blocks (sub-blocks
+// 2h and 2h+1 of a 64-row block, same 16 columns), into eight half2 bit patterns
 //   out[4*kk + 0..3] = A-fragment registers a0..a3 of sub-block 2h+kk:
 //   a0 = (row g,   cols 2t,2t+1)   a1 = (row g+8, cols 2t,2t+1)
 //   a2 = (row g,   cols 2t+8,2t+9) a3 = (row g+8, cols 2t+8,2t+9)
 // w4a / w4b: the lane's 4-bit words of sub-blocks 2h and 2h+1.
-// w2: the lane's 2-bit word that covers both sub-blocks (e3m2 only).
-// w1: the lane's 1-bit word of the column block, which covers all four sub-blocks (e2m2 only);
-//     h selects its upper (h=0) or lower (h=1) half of the iterations.
-template <int E_BITS>
-FPX_HD void unpack16(uint32_t w4a, uint32_t w4b, uint32_t w2, uint32_t w1, int h, uint32_t out[8]) {
-    const uint32_t nib0 = (w4a >> 4) & 0x0f0f0f0fu, nib1 = w4a & 0x0f0f0f0fu;
-    const uint32_t nib2 = (w4b >> 4) & 0x0f0f0f0fu, nib3 = w4b & 0x0f0f0f0fu;
-    uint32_t y0, y1, y2, y3;
-    if (E_BITS == 3) {
-        // iteration n' (0..3) has the sign at bit 7-2n' and e2 at bit 6-2n' of every byte of w2
-        y0 = stitch_e3m2(w2, w2 >> 2, nib0);
-        y1 = stitch_e3m2(w2 << 2, w2, nib1);
-        y2 = stitch_e3m2(w2 << 4, w2 << 2, nib2);
-        y3 = stitch_e3m2(w2 << 6, w2 << 4, nib3);
-    } else {
-        // iteration i (0..7) of the column block has the sign at bit 7-i; this lane pair uses 4h..4h+3
-        const uint32_t s = w1 << (4 * h);
-        y0 = stitch_e2m2(s, nib0);
-        y1 = stitch_e2m2(s << 1, nib1);
-        y2 = stitch_e2m2(s << 2, nib2);
-        y3 = stitch_e2m2(s << 3, nib3);
-    }
-    out[0] = expand_13(y0); out[1] = expand_02(y0); out[2] = expand_13(y1); out[3] = expand_02(y1);
-    out[4] = expand_13(y2); out[5] = expand_02(y2); out[6] = expand_13(y3); out[7] = expand_02(y3);
-}
+// w2: the lane's 2-bit word that covers both sub-blocks (six-bit formats only): of iteration n' (0..3), bits 7-2n' and 6-2n'
+//     of every byte.
+// w1: the lane's 1-bit word of the column block, which covers all four sub-blocks (five-bit formats only): of iteration i
+//     (0..7) bit 7-i of every byte; h selects its upper (h=0) or lower (h=1) half of the iterations.
 
 // The general case: any format whose code is at most 6 bits wide (e2m1, e3m1, e2m3 besides the two above).  Every
 // byte first receives its code left-aligned, [code | 0...], the way the reference's dequantiser assembles it
 // (utils_parallel_dequant.cuh:63-86: the 1-, 2- and 4-bit segments are masked at the top of each byte and shifted
 // right by the width of the segments above them); the bytes are then spread into 16-bit lanes and everything but
 // the sign is shifted right by 5 - E (FPx_FP16_Cast_4Way, :13-28).  About twice the instructions of the two
-// sequences above, which exist because e3m2 and e2m2 are the formats that matter.
+// sequences below, which exist because e3m2 and e2m2 are the formats that matter.
 template <int E_BITS, int M_BITS>
 FPX_HD void unpack16_generic(uint32_t w4a, uint32_t w4b, uint32_t w2, uint32_t w1, int h, uint32_t out[8]) {
     constexpr int BW = 1 + E_BITS + M_BITS;
@@ -175,16 +145,9 @@ FPX_HD void unpack16_generic(uint32_t w4a, uint32_t w4b, uint32_t w2, uint32_t w
     }
 }
 
-// What the kernels call: the short sequences for e3m2 / e2m2, the general one otherwise.
-template <int E_BITS, int M_BITS>
-FPX_HD void unpack16_any(uint32_t w4a, uint32_t w4b, uint32_t w2, uint32_t w1, int h, uint32_t out[8]) {
-    if (M_BITS == 2 && (E_BITS == 3 || E_BITS == 2)) unpack16<(M_BITS == 2 && E_BITS == 2) ? 2 : 3>(w4a, w4b, w2, w1, h, out);
-    else unpack16_generic<E_BITS, M_BITS>(w4a, w4b, w2, w1, h, out);
-}
-
-// The same unpack for the GEMM's inner loop, in fewer instructions and with part of them moved off the logic pipe.
+// e3m2 and e2m2 in the GEMM's inner loop: fewer instructions, and part of them moved off the logic pipe.
 // On B200 the logic operations (LOP3, PRMT, funnel shifts) issue at 64 lanes per clock and SM, and integer
-// multiply-adds issue at the same rate on the other (FMA) pipe; the sequence above keeps only the logic pipe busy.
+// multiply-adds issue at the same rate on the other (FMA) pipe, which shifts and masks alone leave idle.
 // Here the sign and exponent bits are brought into one word once, the left shifts are multiplications, and the low
 // nibbles are what is left of the word after the high ones (w - 16 * high).  The multipliers come in through `k`
 // (kernel parameters on the device), so that the compiler cannot turn them back into shifts; the values are fixed:

@@ -60,7 +60,8 @@ constexpr int kNatFirstIssuer = 2;             // warps 2..5: MMA issue (the fir
 constexpr int kNatMaxIssuers = 4;
 constexpr int kNatFirstEpilogue = kNatFirstIssuer + kNatMaxIssuers;   // warps 6..9: one per tensor-memory lane quadrant
 constexpr int kNatFirstConverter = kNatFirstEpilogue + 4;   // warps 10..: split the fp16 activations (fused variant only)
-constexpr uint32_t kNatPrefetch = 12;           // tiles of a CTA asked into L2 before the previous kernel has finished
+constexpr uint32_t kNatPrefetch = 12;           // tiles of a CTA asked into L2 before the previous kernel has finished: the deepest
+                                                // ring (up to 8 tokens; the rings of wider batches hold fewer, down to 4 stages)
 constexpr int kNatMaxTokens = 64;               // 4 x 64 = 256 MMA columns
 
 template <int N_TILE>
@@ -377,7 +378,7 @@ fpx_native_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         // ------------------------------------------------------------ epilogue: one warp per tensor-memory lane quadrant
         const int q = warp & 3;
         // The first tiles are asked into L2 while the previous kernel of the stream finishes (L2 is where that kernel's stores end
-        // up too, so this reads nothing early): a ring's worth, by the warps that have nothing to do yet.  At one token
+        // up too, so this reads nothing early): kNatPrefetch of them, by the warps that have nothing to do yet.  At one token
         // 22016 x 4096 15.2 -> 13.8 us, 4096 x 11008 9.6 -> 8.7 us; at 16 tokens 57344 x 8192 60.5 -> 56.8 us.
         if (!p.weights_static) {
             SegmentIter ahead;

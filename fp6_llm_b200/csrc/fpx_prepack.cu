@@ -4,8 +4,8 @@
 //                         (fp6_llm/csrc/utils/weight_prepacking.h:118-196);
 //   * dequant (unpacked): the reference's CPU dequantiser on the GPU
 //                         (fp6_llm/csrc/utils/weight_dequant.h:10-48);
-//   * dequant (packed):   prepacked weights -> fp16 [M, K] with exactly the unpack code of the GEMM,
-//                         for fp16 GEMM comparisons and for checking the packed format end to end.
+//   * dequant (packed):   prepacked weights -> fp16 [M, K], for fp16 GEMM comparisons and for checking the packed
+//                         format end to end (by the packers' way backwards, fpx_codes.cuh, not by the GEMM's unpack code);
 //   * repack:             prepacked weights -> the 128 x 128 tiles of fpx_native.cu;
 //   * quantise:           fp16 weights -> row scales, and fp16 weights + row scales -> prepacked weights.
 // All are byte shuffles bounded by HBM traffic (bytes in + bytes out).

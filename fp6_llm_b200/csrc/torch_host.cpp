@@ -53,7 +53,7 @@ bool whole(PyObject* o, long* v) {
 }
 
 struct Call {
-    int e = 0, m = 0, split_k = 0, activation = 0;
+    int e = 0, m = 0, activation = 0;
     const at::Tensor *x = nullptr, *weight = nullptr, *native = nullptr, *scales = nullptr, *bias = nullptr;
 };
 
@@ -103,7 +103,7 @@ PyObject* run(const Call& c, bool last_dim_only) {
             return not_mine();
     } else {
         const at::Tensor& w = *c.weight;
-        if (w.dim() != 2 || w.size(0) != oc || w.size(1) * 32 != ic * (1 + c.e + c.m) || c.split_k < 0) return not_mine();
+        if (w.dim() != 2 || w.size(0) != oc || w.size(1) * 32 != ic * (1 + c.e + c.m)) return not_mine();
     }
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     c10::DimVector sizes(x.sizes());
@@ -147,14 +147,13 @@ bool common(Call* c, PyObject* e, PyObject* m, PyObject* x, PyObject* scales, Py
     return bias == Py_None || (c->bias = plain(bias, at::kHalf, device));
 }
 
-// linear(e, m, x, packed, scales, split_k, bias, activation)
+// linear(e, m, x, packed, scales, split_k, bias, activation); split_k is checked, how K is split is the library's choice
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     Call c;
     long split;
     if (n != 8 || !whole(a[5], &split) || split < 0 || split > 65535 || !common(&c, a[0], a[1], a[2], a[4], a[6], a[7])) return not_mine();
     if (!(c.weight = plain(a[3], at::kInt, c.x->get_device()))) return not_mine();
-    c.split_k = (int)split;
     return run(c, false);
     END_HANDLE_TH_ERRORS
 }
@@ -170,7 +169,7 @@ PyObject* native(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // layer(e, m, x, packed, tiles or None, scales, split_k, bias, activation): the modules' forward, x of any rank; the tile
-// layout is taken when the library prefers it for this batch
+// layout is taken when the library prefers it for this batch and split_k is 0, which is all that split_k says
 PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     Call c;
@@ -178,7 +177,6 @@ PyObject* layer(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != 9 || !whole(a[6], &split) || split < 0 || split > 65535 || !common(&c, a[0], a[1], a[2], a[5], a[7], a[8])) return not_mine();
     const int device = c.x->get_device();
     if (!(c.weight = plain(a[3], at::kInt, device))) return not_mine();
-    c.split_k = (int)split;
     const int64_t dim = c.x->dim(), oc = c.scales->numel();
     const int64_t ic = dim ? c.x->size(dim - 1) : 0;
     if (ic < 64 || c.weight->dim() != 2 || c.weight->size(0) != oc || c.weight->size(1) * 32 != ic * (1 + c.e + c.m)) return not_mine();

@@ -38,7 +38,8 @@ def HeuristicFuntion_SplitK(M, N, Num_GPU_SMs):
 
 
 def heuristic_split_k_b200(M: int, N: int, K: int, num_sms: int = 148) -> int:
-    """Split-K for the sm_100a kernel: 128-row tiles, one CTA per SM, K-aware (C: fp6b200_choose_split_k)."""
+    """Split-K for the sm_100a kernel: 128-row tiles, one CTA per SM, K-aware (C: fp6b200_choose_split_k).  For C callers that bring
+    a split and its workspace; the Python operators split K as the library finds best, whatever split they are given."""
     return int(_native.lib().fp6b200_choose_split_k(M, N, K, num_sms))
 
 

@@ -145,7 +145,8 @@ int fp6b200_kernel_launches(size_t M, size_t N, size_t K, int split_k);
  * Split count for callers that keep the reference's explicit split-K scheme: the best split_k >= 1 for this
  * kernel on a GPU with `num_sms` SMs (148 on B200), given its 128-row tiles, one CTA per SM and the K blocks
  * available.  The reference's own heuristic (HeuristicFuntion_SplitK, fp6_llm/__init__.py:13-23) is kept
- * separately, unchanged, in Python.  Passing split_k = 0 to fp6b200_linear is usually faster than either.
+ * separately, unchanged, in Python.  Passing split_k = 0 to fp6b200_linear is usually faster than either, and a split
+ * >= 1 only decides what runs where its workspace is too small for the library's own decomposition (see fp6b200_linear).
  */
 int fp6b200_choose_split_k(size_t M, size_t N, size_t K, int num_sms);
 
@@ -249,8 +250,9 @@ int fp6b200_linear_gather(int e_bits, int m_bits, void* stream, const void* weig
  * FP6B200_OPTION_STATIC_WEIGHTS (default 0): set to 1 to promise that no packed-weight buffer handed to fp6b200_linear*
  * is written by work that is still in flight on the same stream when the call is made (weights prepacked at load time
  * and then only read).  The GEMM is launched programmatically: its CTAs start while the previous kernel of the stream
- * is finishing, and with this option they already request the first weight stages and unpack them then; activations,
- * scales, outputs and workspace are touched only after the previous kernel has completed, option or not.
+ * is finishing, and with this option they already request the first weight stages and unpack them then (without it they may
+ * ask L2 for them, which reads nothing early); activations, scales, outputs and workspace are touched only after the previous
+ * kernel has completed, option or not.
  * With the option on, a prepack (or any write of the weights) must be followed by a synchronisation or an event wait
  * before the first GEMM that reads them.  fp6b200_set_option returns cudaErrorInvalidValue for an unknown option;
  * fp6b200_get_option returns the value, or -1.

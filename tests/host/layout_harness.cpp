@@ -35,7 +35,7 @@ int harness_prepack(int e_bits, int m_bits, uint8_t* out, const uint8_t* in, uin
 }
 
 // The GEMM's unpack path: for every 128-row tile, 64-wide K block, tensor-memory quadrant q and lane, read
-// the words the kernel reads (stage layout = [segment][row block][word]), run unpack16 and scatter the
+// the words the kernel reads (stage layout = [segment][row block][word]), run the kernel's unpack and scatter the
 // registers the way tcgen05.st.16x128b.x8 places them (thread 4g+t, register 2c+hr -> lane g+8hr, 32-bit
 // column t+4c).  out_bits[row*cols+col] receives the unscaled fp16 pattern.
 int harness_unpack(int e_bits, int m_bits, uint16_t* out_bits, const uint8_t* packed, uint32_t rows, uint32_t cols) {
@@ -59,20 +59,13 @@ int harness_unpack(int e_bits, int m_bits, uint16_t* out_bits, const uint8_t* pa
                         uint32_t pat[8];
                         uint32_t pat2[8];
                         const UnpackMul km = unpack_mul_values(h);
-                        if (m_bits == 2 && e_bits == 3) {
-                            unpack16<3>(w4a, w4b, w2, w1, h, pat);
-                            unpack16_mul<3>(w4a, w4b, w2, w1, km, pat2);      // the GEMM's multiply-based sequence: same registers
-                            for (int i = 0; i < 8; i++) if (pat[i] != pat2[i]) return -2;
-                            unpack16_generic<3, 2>(w4a, w4b, w2, w1, h, pat2);   // and so must the general sequence
-                        } else if (m_bits == 2 && e_bits == 2) {
-                            unpack16<2>(w4a, w4b, w2, w1, h, pat);
-                            unpack16_mul<2>(w4a, w4b, w2, w1, km, pat2);
-                            for (int i = 0; i < 8; i++) if (pat[i] != pat2[i]) return -2;
-                            unpack16_generic<2, 2>(w4a, w4b, w2, w1, h, pat2);
-                        } else if (e_bits == 2 && m_bits == 1) { unpack16_any<2, 1>(w4a, w4b, w2, w1, h, pat); unpack16_generic<2, 1>(w4a, w4b, w2, w1, h, pat2); }
-                        else if (e_bits == 3 && m_bits == 1) { unpack16_any<3, 1>(w4a, w4b, w2, w1, h, pat); unpack16_generic<3, 1>(w4a, w4b, w2, w1, h, pat2); }
-                        else { unpack16_any<2, 3>(w4a, w4b, w2, w1, h, pat); unpack16_generic<2, 3>(w4a, w4b, w2, w1, h, pat2); }
-                        for (int i = 0; i < 8; i++) if (pat[i] != pat2[i]) return -3;
+                        // e3m2 and e2m2 run the multiply-based sequence, the other formats the general one, which must agree
+                        if (e_bits == 3 && m_bits == 2) { unpack16_mul<3>(w4a, w4b, w2, w1, km, pat); unpack16_generic<3, 2>(w4a, w4b, w2, w1, h, pat2); }
+                        else if (e_bits == 2 && m_bits == 2) { unpack16_mul<2>(w4a, w4b, w2, w1, km, pat); unpack16_generic<2, 2>(w4a, w4b, w2, w1, h, pat2); }
+                        else if (e_bits == 2 && m_bits == 1) unpack16_generic<2, 1>(w4a, w4b, w2, w1, h, pat);
+                        else if (e_bits == 3 && m_bits == 1) unpack16_generic<3, 1>(w4a, w4b, w2, w1, h, pat);
+                        else unpack16_generic<2, 3>(w4a, w4b, w2, w1, h, pat);
+                        if (m_bits == 2) for (int i = 0; i < 8; i++) if (pat[i] != pat2[i]) return -2;
                         for (int kk = 0; kk < 2; kk++)
                             for (int i = 0; i < 4; i++) v[kk][4 * j + i] = pat[4 * kk + i];
                     }

@@ -1,8 +1,8 @@
 """GPU parity of the linear layer on the shapes and batch sizes the benchmark workloads are quoted on.
 
 Against the oracle (reference dequantisation + fp32 matmul) on row slices that keep the FULL K and the full batch-size
-set of every workload: LLaMA-2-7B FP6 (K 4096 / 11008), LLaMA-2-13B FP5 (K 5120 / 13824, explicit split-K 1/2/4/8 and
-the library's own decomposition), LLaMA-2-70B FP6 (K 8192 / 28672, batch 1..128) and the prefill batches 512..2048.
+set of every workload: LLaMA-2-7B FP6 (K 4096 / 11008), LLaMA-2-13B FP5 (K 5120 / 13824, called with splitK 1/2/4/8 and 0,
+which all run the library's own decomposition), LLaMA-2-70B FP6 (K 8192 / 28672, batch 1..128) and the prefill batches 512..2048.
 At the FULL layer shapes the oracle is too slow, so every (layer, batch) pair of the 70B workloads is checked per block
 of 32 output channels against an fp32 matmul on the GPU-dequantised weights (that dequantiser is bit-exact against the
 oracle, see test_gpu_formats.py).  Tolerances as in test_gpu_linear.py."""

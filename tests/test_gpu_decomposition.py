@@ -50,7 +50,8 @@ def test_every_decomposition(oc, ic, bs):
 @pytest.mark.parametrize("oc,ic,bs", [(512, 1088, 5), (4096, 704, 16), (1280, 5120, 70), (19200, 2048, 3), (768, 2048, 300)])
 @pytest.mark.parametrize("split_k", [1, 2, 3, 12, 40])
 def test_callers_split_stays_in_its_workspace(native_lib, oc, ic, bs, split_k):
-    """split_k * M * N floats are what the caller owns, whatever decomposition runs; none for split_k = 1."""
+    """split_k * M * N floats are what the caller owns, whatever decomposition runs; none for split_k = 1.  (All of these fit the
+    library's own; test_callers_split_runs_as_asked has shapes that do not.)"""
     import fp6_llm_b200 as f
     packed, s, x, _, plain = _layer(oc, ic, bs, 2, 2)
     elems = split_k * oc * bs if split_k > 1 else 0

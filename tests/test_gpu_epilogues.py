@@ -1,6 +1,7 @@
 """The fused epilogues of fp6b200_linear_ex (bias in fp32, silu(gate) * up on interleaved rows) against the oracle's
-linear layer followed by the same arithmetic in fp32 on the CPU; every path a tile can take to memory: stored by the
-GEMM, summed by the stream-K fix-up, summed by the split-K reduction.  Tolerances of the linear layer."""
+linear layer followed by the same arithmetic in fp32 on the CPU; through the operators, whose tiles are stored by the GEMM, by a
+cluster or by the stream-K fix-up (the split-K reduction is the C interface's: test_gpu_decomposition.py).  Tolerances of
+the linear layer."""
 import numpy as np
 import pytest
 import torch
@@ -29,7 +30,7 @@ def _close(oracle_mod, y, truth):
     assert res["rel_fro"] <= REL_FRO and res["max_row_rel"] <= ROW_MAX, res
 
 
-# (oc, ic, bs, split_k): direct tiles only; stream-K with a fix-up; explicit split-K with the reduction kernel; wide tiles
+# (oc, ic, bs, split_k): few tokens, many, wide and two token tiles; the split is accepted, the library's choice runs
 SHAPES = [(512, 1024, 8, 1), (4096, 2048, 12, 0), (1536, 4096, 40, 0), (512, 2048, 33, 4), (768, 1024, 130, 0), (512, 1024, 300, 2)]
 
 

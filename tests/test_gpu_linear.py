@@ -46,7 +46,8 @@ def test_batch_sweep_fp6(oracle_mod, bs):
 @pytest.mark.parametrize("e,m", FORMATS)
 @pytest.mark.parametrize("split_k", [1, 2, 3, 7, 8, 11, 0])
 def test_split_k(oracle_mod, e, m, split_k):
-    """K = 512 has 8 K-blocks: uneven splits, one block per split, more splits than blocks, and the library's choice."""
+    """K = 512 has 8 K-blocks: every splitK a program may pass is taken, and how K is split is the library's choice for all of
+    them (the split as asked is the C interface's: test_gpu_decomposition.py)."""
     import fp6_llm_b200 as f
     packed, s, x, truth = _case(oracle_mod, e, m, 256, 512, 12, seed=split_k + e)
     _check(oracle_mod, f.linear_forward_eXmY_cuda(e, m, x, packed, s, split_k), truth)
@@ -114,7 +115,7 @@ def test_weights_written_just_before(bs, native):
 @pytest.mark.parametrize("split_k", [0, 1, 3])
 def test_tile_widths(oracle_mod, bs, split_k):
     """Batches are cut into equally wide token tiles of any multiple of 16 columns: the last token of a tile, the first of the
-    next, and widths at both ends of every kernel's range, for whole tiles, stream-K slots and the caller's split."""
+    next, and widths at both ends of every kernel's range, whatever splitK the call names."""
     import fp6_llm_b200 as f
     packed, s, x, truth = _case(oracle_mod, 2, 2, 512, 704, bs, seed=bs)
     _check(oracle_mod, f.linear_forward_eXmY_cuda(2, 2, x, packed, s, split_k), truth)
