@@ -1074,8 +1074,9 @@ int make_plan(size_t M, size_t n_tiles, size_t K, int split_k, int sms, const Pl
             const uint64_t waves = tiles / (clusters * c), rem = tiles - waves * clusters * c;
             if (rem > clusters || rem == 0) continue;
             // with waves before it, a size that does not divide the SM groups evenly waits for its SMs to come free together:
-            // 57344 x 8192 on the native path, three against two: 61.5 and 57.9 us at 16 tokens, 108.9 and 102.4 at 64 (the one layer
-            // where the costs would have picked three; five, six and seven go with it unmeasured)
+            // three against two on the native path 57344 x 8192 61.5 and 57.9 us at 16 tokens, 108.9 and 102.4 at 64, 22016 x 4096 15.2 and
+            // 13.1 at one token, 31.0 and 26.0 at 64; on this path 57344 x 8192 208.5 and 180.7 at 256, 22016 x 4096 29.9 and 29.6 at 128
+            // (22.9 and 23.9 at 64, the one case for three).  Five, six and seven go with it: no layer measured leaves them room.
             if (waves && (c & (c - 1))) continue;
             const double cost = phase(kb * (double)waves, (double)(waves * clusters * c) * kb) +
                                 phase((double)((plan.kblocks + c - 1) / c), (double)rem * kb) + costs.reduce + (waves ? costs.segment : 0.0);
