@@ -191,7 +191,7 @@ def lib() -> ctypes.CDLL:
 
 class _PythonForm:
     """Stands in for the extension: every call is left to the Python form of the same operator."""
-    linear = native = layer = host_batch = staticmethod(lambda *args: NotImplemented)
+    linear = native = layer = host_batch = unwatched = staticmethod(lambda *args: NotImplemented)
 
 
 _host = None

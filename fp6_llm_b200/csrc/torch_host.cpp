@@ -10,9 +10,13 @@
 // argument) is left to the Python form of the same operator, which converts or raises.
 #include <Python.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/TracerMode.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <c10/core/DispatchKeySet.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -237,7 +241,20 @@ PyObject* host_batch(PyObject*, PyObject* calls) {
     END_HANDLE_TH_ERRORS
 }
 
+// unwatched(t): ops.is_plain_memory without its calls into Python, which took 3 us of the 80 of a small layer's loading
+PyObject* unwatched(PyObject*, PyObject* o) {
+    HANDLE_TH_ERRORS
+    if (at::impl::PythonTorchFunctionTLS::stack_len() != 0) return not_mine();   // which modes these are is known in Python
+    if (!THPVariable_CheckExact(o)) Py_RETURN_FALSE;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    const bool watched = t.key_set().has_any(kWrapped) || (t.requires_grad() && c10::GradMode::is_enabled()) || t._fw_grad(0).defined() ||
+                         c10::impl::TorchDispatchModeTLS::any_modes_set() || at::tracer::impl::is_dispatch_enabled();
+    return PyBool_FromLong(!watched);
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"unwatched", unwatched, METH_O, nullptr},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(linear)), METH_FASTCALL, nullptr},
     {"native", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(native)), METH_FASTCALL, nullptr},
     {"layer", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(layer)), METH_FASTCALL, nullptr},

@@ -11,8 +11,8 @@ import torch
 
 from . import _native
 from .formats import bit_width, check_format, magnitudes
-from .ops import (ACT_NONE, ACT_SILU_MUL, interleave_gate_up, is_plain_memory, linear_forward_ex, linear_forward_native,
-                  native_preferred, native_repack, native_supported, quantize_prepack_cuda, row_scales_cuda)
+from .ops import (ACT_NONE, ACT_SILU_MUL, interleave_gate_up, is_plain_memory, launch_row_scales, linear_forward_ex,
+                  linear_forward_native, native_preferred, native_repack, native_supported, quantize_prepack_cuda)
 
 
 def _enable_native(layer) -> None:
@@ -22,21 +22,16 @@ def _enable_native(layer) -> None:
     layer.register_buffer("weight_native", native_repack(layer.e_bits, layer.m_bits, layer.weight))
 
 
-def _held(layer, name: str):
-    """What `layer.name` gives, None if there is none, without Module.__getattr__ where that can be helped: a lookup through it
-    costs 0.5 us, a failing one 1.6 us.  A program may have put a Parameter, a plain attribute or a property of a subclass in a
-    buffer's place (assigning a Parameter takes the name out of the buffers)."""
-    fields = layer.__dict__
-    if name in fields["_buffers"] and name not in fields:
-        return fields["_buffers"][name]
-    if name in fields or name in fields["_parameters"] or hasattr(type(layer), name):
-        return getattr(layer, name)
-    return None
-
-
 def _forward(layer, x: torch.Tensor, activation: int) -> torch.Tensor:
-    y = _native.host().layer(layer.e_bits, layer.m_bits, x, _held(layer, "weight"), _held(layer, "weight_native"),
-                             _held(layer, "scales"), layer.split_k, _held(layer, "bias"), activation)
+    # From the buffers' own dict: a lookup through Module.__getattr__ costs 0.5 us, a failing one 1.6 us.  A program may have put
+    # something else in a buffer's place (assigning a Parameter takes the name out of the buffers).  A weight or scales that are
+    # not found there make the binding decline; no bias is a valid call, so a bias that is not there is looked up.
+    held = layer._buffers
+    tiles = held.get("weight_native")
+    if tiles is None:
+        tiles = layer._parameters.get("weight_native")
+    y = _native.host().layer(layer.e_bits, layer.m_bits, x, held.get("weight"), tiles, held.get("scales"), layer.split_k,
+                             held["bias"] if "bias" in held else layer.bias, activation)
     if y is not NotImplemented:   # the native host side took the call: contiguous fp16 activations on the weights' device
         return y
     if x.dtype != torch.float16 or x.shape[-1] != layer.in_features:
@@ -78,7 +73,7 @@ class FPxLinear(torch.nn.Module):
         top = float(magnitudes(e_bits, m_bits)[-1])
         if (weight.is_cuda and weight.dtype == torch.float16 and weight.dim() == 2 and is_plain_memory(weight) and weight.is_contiguous()
                 and weight.numel() and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0):
-            return row_scales_cuda(weight, top)
+            return launch_row_scales(weight, top)
         return (weight.float().abs().amax(dim=1) / top).clamp_min(2.0 ** -24).to(torch.float16)
 
     @classmethod

@@ -11,6 +11,7 @@ import math
 import operator
 
 import torch
+from torch.autograd import forward_ad
 from torch.overrides import _get_current_function_mode_stack
 from torch.utils._device import DeviceContext
 
@@ -331,14 +332,20 @@ def is_plain_memory(t: torch.Tensor) -> bool:
     """Whether a kernel that reads t's memory may stand in for tensor operations on t: nothing records the operations (autograd
     in reverse or forward mode, tracing, an active mode) and t is not a wrapper around something else (a tensor subclass, vmap and
     the other function transforms, a lazily negated view)."""
-    return (type(t) in (torch.Tensor, torch.nn.Parameter)
+    if torch.compiler.is_compiling():
+        return False
+    plain = _native.host().unwatched(t)
+    if plain is not NotImplemented:
+        return plain
+    kind = type(t)
+    return ((kind is torch.Tensor or kind is torch.nn.Parameter)
             and not (t.requires_grad and torch.is_grad_enabled())
-            and not torch._C._functorch.is_functorch_wrapped_tensor(t)
-            and not t.is_neg() and not torch._is_zerotensor(t)
-            and torch.autograd.forward_ad.unpack_dual(t).tangent is None
+            and not torch._C._functorch.is_functorch_wrapped_tensor(t) and not t.is_neg() and not torch._is_zerotensor(t)
+            and (forward_ad._current_level < 0 or forward_ad.unpack_dual(t).tangent is None)
             and torch._C._len_torch_dispatch_stack() == 0
-            and all(isinstance(mode, DeviceContext) for mode in _get_current_function_mode_stack())   # `with torch.device(..)` is none
-            and not torch.jit.is_tracing() and not torch.compiler.is_compiling())
+            and (torch._C._len_torch_function_stack() == 0   # `with torch.device(..)` is a mode that records nothing
+                 or all(isinstance(mode, DeviceContext) for mode in _get_current_function_mode_stack()))
+            and torch._C._get_tracing_state() is None)
 
 
 def row_scales_cuda(weights: torch.Tensor, top: float) -> torch.Tensor:
@@ -346,6 +353,11 @@ def row_scales_cuda(weights: torch.Tensor, top: float) -> torch.Tensor:
     `top`, at least 2^-24, in one pass over the weights (C: fp6b200_row_scales; no counterpart in the reference)."""
     if not weights.is_cuda or weights.dtype != torch.float16 or weights.dim() != 2 or not weights.is_contiguous():
         raise ValueError("expected a contiguous fp16 CUDA tensor [OC, IC]")
+    return launch_row_scales(weights, top)
+
+
+def launch_row_scales(weights: torch.Tensor, top: float) -> torch.Tensor:
+    """:func:`row_scales_cuda` for a caller that has checked the tensor."""
     OC, IC = weights.shape
     out = torch.empty(OC, dtype=torch.float16, device=weights.device)
     with torch.cuda.device(weights.device):

@@ -78,10 +78,56 @@ def test_row_scales_of_tensors_without_memory():
     got = FPxLinear.row_scales(fake, 3, 2)
     assert got.shape == (64,) and got.dtype == torch.float16 and got.device.type == "cuda"
     w = torch.randn(4, 8).half()
-    assert is_plain_memory(w) and is_plain_memory(torch.nn.Parameter(w, requires_grad=False))
-    assert not is_plain_memory(torch.nn.Parameter(w)) and not is_plain_memory(torch._neg_view(w))
-    with torch.no_grad():
-        assert is_plain_memory(torch.nn.Parameter(w))
     for bad in (w, fake.float(), fake.t(), fake[0]):
         with pytest.raises(ValueError):
             row_scales_cuda(bad, 28.0)
+
+
+def test_what_is_plain_memory(native_lib, monkeypatch):
+    """The native answer and the Python form of it."""
+    import torch
+    from torch.autograd import forward_ad
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from fp6_llm_b200 import _native
+    from fp6_llm_b200.ops import is_plain_memory as plain
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, fn, types, args=(), kwargs=None):
+            return fn(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, fn, types, args=(), kwargs=None):
+            return fn(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+
+    w = torch.randn(4, 8).half()
+    with FakeTensorMode():
+        fake = torch.empty(4, 8)
+    for form in (_native.host(), _native._PythonForm):
+        monkeypatch.setattr(_native, "_host", form)
+        assert plain(w) and plain(torch.nn.Parameter(w, requires_grad=False)) and plain(w[1:, ::2])
+        assert not any(map(plain, (torch.nn.Parameter(w), torch._neg_view(w), fake, w.as_subclass(Sub), torch._efficientzerotensor(4, 4))))
+        with torch.no_grad():
+            assert plain(torch.nn.Parameter(w))
+        with torch.inference_mode():
+            assert plain(w.clone())
+        with forward_ad.dual_level():
+            assert plain(w) and not plain(forward_ad.make_dual(w, w))
+        with Dispatch():
+            assert not plain(w)
+        with Function():
+            assert not plain(w)
+        with torch.device("cpu"):
+            assert plain(w) and not plain(torch._neg_view(w))
+        seen = []
+        look = lambda t: (seen.append(plain(t)), t.float().sum())[1]   # noqa: E731
+        torch.func.vmap(look)(w)
+        torch.func.grad(look)(w)
+        torch.func.jvp(look, (w,), (w,))
+        torch.func.functionalize(look)(w)
+        torch.jit.trace(look, (w,), check_trace=False)
+        assert seen == [False] * 5 and plain(w)
