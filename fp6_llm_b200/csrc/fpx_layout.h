@@ -118,12 +118,12 @@ FPX_HD uint32_t expand_02(uint32_t y) {   // bytes 2,0 -> high bytes of the two 
 // w1: the lane's 1-bit word of the column block, which covers all four sub-blocks (five-bit formats only): of iteration i
 //     (0..7) bit 7-i of every byte; h selects its upper (h=0) or lower (h=1) half of the iterations.
 
-// The general case: any format whose code is at most 6 bits wide (e2m1, e3m1, e2m3 besides the two above).  Every
+// The general case: any format whose code is at most 6 bits wide (e2m1, e3m1, e2m3 besides e3m2 and e2m2).  Every
 // byte first receives its code left-aligned, [code | 0...], the way the reference's dequantiser assembles it
 // (utils_parallel_dequant.cuh:63-86: the 1-, 2- and 4-bit segments are masked at the top of each byte and shifted
 // right by the width of the segments above them); the bytes are then spread into 16-bit lanes and everything but
 // the sign is shifted right by 5 - E (FPx_FP16_Cast_4Way, :13-28).  About twice the instructions of the two
-// sequences below, which exist because e3m2 and e2m2 are the formats that matter.
+// sequences of unpack16_mul, which exist because e3m2 and e2m2 are the formats that matter.
 template <int E_BITS, int M_BITS>
 FPX_HD void unpack16_generic(uint32_t w4a, uint32_t w4b, uint32_t w2, uint32_t w1, int h, uint32_t out[8]) {
     constexpr int BW = 1 + E_BITS + M_BITS;
